@@ -134,6 +134,7 @@ def lib() -> C.CDLL:
         "dns_plane_stats": (I, [P, P]),
         "dns_set_profiling": (I, [P, I]),
         "dns_kernel_times": (I, [P, P, P]),
+        "dns_set_fine_pairs": (I, [P, I]),
         "dns_batch_create": (I, [I, C.POINTER(P)]),
         "dns_batch_destroy": (None, [P]),
         "dns_batch_footprint": (I, [C.POINTER(Params), C.POINTER(C.c_longlong)]),
@@ -312,6 +313,10 @@ class Channel:
     # ---- measurement
     def set_profiling(self, on: bool):
         _check(lib().dns_set_profiling(self.h, 1 if on else 0), "dns_set_profiling")
+
+    def set_fine_pairs(self, mode: int):
+        """Two fine substeps a pass: -1 by size (default), 0 never, 1 wherever possible."""
+        _check(lib().dns_set_fine_pairs(self.h, mode), "dns_set_fine_pairs")
 
     def kernel_times(self):
         """{kernel class: (total ms, launches)} since profiling was switched on."""

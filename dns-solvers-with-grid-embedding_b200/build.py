@@ -2,7 +2,7 @@
 programs ``dns_run`` (the solver) and ``dns_budget`` (the budget analysis),
 plain C over the library's C ABI.
 
-``kernels_f64.cu`` is compiled with ``-fmad=false``: the FP64 plain form must
+``kernels_f64.cu`` and ``pair_f64.cu`` are compiled with ``-fmad=false``: the FP64 plain form must
 not fuse multiply-adds, so that its per-node arithmetic rounds exactly like the
 reference.  ``tke.cu`` (the statistics / budget analysis) likewise.  Everything else uses the default flags.  Run
 ``python build.py`` (or call ``build()``); nvcc cross-compiles without a GPU.
@@ -24,6 +24,7 @@ ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-I", str(INCLUDE), "-I", str(CSRC)]
 UNITS = {  # source -> extra flags
     "kernels_f64.cu": ["-fmad=false"],
+    "pair_f64.cu": ["-fmad=false"],
     "kernels_f32.cu": [],
     "batch_f32.cu": [],
     "dns_api.cu": [],

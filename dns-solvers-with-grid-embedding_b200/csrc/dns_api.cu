@@ -70,7 +70,8 @@ struct dns_handle {
   DevLog *dlog = nullptr;              // kLogCap rows
   DevLog *hlog = nullptr;              // pinned mirror
   double *stats_acc = nullptr;         // [nz_profile][kStatRow] running statistics
-  double *iface_mac = nullptr;         // FP64: interface rho, u [2][4][nyf][nxf]; FP32: corner data
+  double *iface_mac = nullptr;         // FP64: interface rho, u [GR][2][4][nyf][nxf]; FP32: corner data
+  double *iface_mid = nullptr;         // interface planes between the substeps of a pass [GR / 2][2][19][nyf][nxf]
   void *tke_ws = nullptr;              // statistics / budget work space (allocated on first use)
   size_t tke_ws_bytes = 0;
   double *tke_wall = nullptr;          // planar fields of the two wall planes [2][4][nyf][nxf]
@@ -84,6 +85,7 @@ struct dns_handle {
   long ss = 0;                         // coarse steps since load / seed
   int tm = 0;                          // time origin of the log stamps (TSTR or restart counter)
   long sample_every = 0;
+  int pairs = -1;                      // two fine substeps a pass: -1 by size, 0 never, 1 where built
   // Wall-plane populations (the step never reads or writes them; files carry
   // them): wall_dev [2 walls][GR xdv][GR ydv][19] on the device is the primary
   // copy, which the AoS transfers fill and read without a host pass;
@@ -97,7 +99,21 @@ struct dns_handle {
   Profiler prof;
 };
 
-static bool d_gr_ok(const dns_handle *h) { return h->d.gr <= 4; }
+// fine substeps are taken two at a time where the kernels allow it
+static bool pairs_built(const dns_handle *h) { return h->p.precision == DNS_FP64 && h->shape.pair.on(); }
+static bool pairs_on(const dns_handle *h) {
+  return pairs_built(h) && (h->pairs < 0 ? pairs_pay_f64(h->d, h->shape.pair) : h->pairs > 0);
+}
+
+// what the passes of two substeps need beyond the single ones
+static int ready_pairs(dns_handle *h) {
+  if (h->iface_mid) return DNS_OK;
+  const size_t bytes = (h->g.gr / 2) * 2ull * 19 * h->g.nyf * h->g.nxf * (h->p.precision == DNS_FP32 ? 4 : 8);
+  if (prepare_pair_f64()) return fail(DNS_ECUDA, "shared-memory limit of the two-substep kernels");
+  if (cudaMalloc((void **)&h->iface_mid, bytes) != cudaSuccess)
+    return fail(DNS_ENOMEM, "interface planes between two substeps");
+  return DNS_OK;
+}
 
 // Bracket one launch with events when profiling; returns the pair index or -1.
 static int prof_begin(dns_handle *h, int cls) {
@@ -267,8 +283,9 @@ extern "C" int dns_geometry_of(const dns_params *p, dns_geometry *g) {
   PartialLayout pl = partial_layout(d, s);
   const long long nc = 19LL * g->nzc * g->ny * g->nx, nf = 19LL * 2 * p->zds * g->nyf * g->nxf;
   const long long esz = p->precision == DNS_FP32 ? 4 : 8;  // bytes per stored population
-  const long long mac = esz == 4 ? 2LL * 23 * g->ny * g->nx * 4 : 8LL * g->nyf * g->nxf;  // elements of esz
-  g->device_bytes = esz * (2 * nc + 2 * nf + 3LL * 2 * 23 * g->ny * g->nx + mac) +
+  const long long mac = esz == 4 ? 2LL * 23 * g->ny * g->nx * 4 : 8LL * GR * g->nyf * g->nxf;  // elements of esz
+  const long long mid = esz == 8 && pairs_pay_f64(d, s.pair) ? (GR / 2) * 2LL * 19 * g->nyf * g->nxf : 0;
+  g->device_bytes = esz * (2 * nc + 2 * nf + 3LL * 2 * 23 * g->ny * g->nx + mac + mid) +
                     8 * (pl.total + (long long)kStatRow * g->nz_profile + 2LL * 19 * g->nyf * g->nxf) +
                     (long long)g->nyf * g->nxf + (long long)kLogCap * sizeof(DevLog) + sizeof(DevState);
   return DNS_OK;
@@ -313,6 +330,7 @@ extern "C" void dns_destroy(dns_handle *h) {
   cudaFree(h->dlog);
   cudaFree(h->stats_acc);
   cudaFree(h->iface_mac);
+  cudaFree(h->iface_mid);
   cudaFree(h->tke_ws);
   cudaFree(h->tke_wall);
   cudaFree(h->wall_dev);
@@ -375,8 +393,12 @@ extern "C" int dns_create(const dns_params *p, dns_handle **out) {
   if ((rc = alloc((void **)&h->dlog, kLogCap * sizeof(DevLog)))) return rc;
   if ((rc = alloc((void **)&h->stats_acc, (size_t)g.nz_profile * kStatRow * 8))) return rc;
   // FP64: interface rho, u at fine nodes; FP32: corner values and derivatives (float4)
-  const size_t mac_bytes = esz == 4 ? 2ull * 23 * g.ny * g.nx * 16 : 8ull * g.nyf * g.nxf * esz;
+  const size_t mac_bytes = esz == 4 ? 2ull * 23 * g.ny * g.nx * 16 : 8ull * g.gr * g.nyf * g.nxf * esz;
   if ((rc = alloc((void **)&h->iface_mac, mac_bytes))) return rc;
+  if (pairs_on(h) && (rc = ready_pairs(h))) {
+    dns_destroy(h);
+    return rc;
+  }
   if ((rc = alloc((void **)&h->fin_counter, 256))) return rc;
   cudaMemset(h->fin_counter, 0, 256);
   if ((rc = alloc((void **)&h->wall_dev, 2ull * g.nxf * g.nyf * 19 * 8))) return rc;
@@ -1117,16 +1139,37 @@ static void L_fine(dns_handle *h, int src, int dst, bool first, bool last, bool 
     launch_fine_f64(h->ff[src], h->ff[dst], h->wflag, h->d, h->shape, h->g.omega_f, h->state, h->partials, h->pl,
                     first, last, stats, st);
 }
-static void L_iface(dns_handle *h, int fbuf, int it, cudaStream_t st) {
+// Two substeps in one pass; m: slot of the interface planes between them
+static void L_fine_pair(dns_handle *h, int src, int dst, int m, bool first, bool last, cudaStream_t st) {
+  const double *mid = h->iface_mid + (size_t)m * 2 * 19 * h->d.nyf * h->d.nxf;
+  launch_fine_pair_f64(h->ff[src], h->ff[dst], mid, h->wflag, h->d, h->shape.pair, h->g.omega_f, h->state,
+                       h->partials + h->pl.fine, h->partials + h->pl.wall, first, last, st);
+}
+// Interface planes of substep it: those of the fine buffer fbuf, or (fbuf < 0)
+// slot m of the planes between two substeps of a pass
+struct IfaceDest {
+  int it, fbuf, m;
+};
+static void L_iface(dns_handle *h, const IfaceDest *to, int n, cudaStream_t st) {
   const size_t hs = hslot_elems(h);
   if (is_f32(h)) {
     float *H = F(h->hist);
-    launch_interface_f32(H + h->hn * hs, H + h->hp * hs, H + h->hpp * hs, F(h->iface_mac), F(h->ff[fbuf]), h->d, it,
-                         h->g.omega_c, h->g.omega_f, st);
-  } else {
-    launch_interface_f64(h->hist + h->hn * hs, h->hist + h->hp * hs, h->hist + h->hpp * hs, h->iface_mac,
-                         h->ff[fbuf], h->d, h->shape, it, h->g.omega_c, h->g.omega_f, st);
+    for (int q = 0; q < n; q++)
+      launch_interface_f32(H + h->hn * hs, H + h->hp * hs, H + h->hpp * hs, F(h->iface_mac), F(h->ff[to[q].fbuf]),
+                           h->d, to[q].it, h->g.omega_c, h->g.omega_f, st);
+    return;
   }
+  const size_t plane = (size_t)h->d.nyf * h->d.nxf;
+  IfaceTarget tg[4];
+  for (int q = 0; q < n; q++) {
+    tg[q].substep = to[q].it;
+    for (int w = 0; w < 2; w++)
+      tg[q].out[w] = to[q].fbuf >= 0 ? h->ff[to[q].fbuf] + (size_t)(h->d.zds - 1 + w) * plane
+                                     : h->iface_mid + (size_t)(to[q].m * 2 + w) * 19 * plane;
+    tg[q].stride = to[q].fbuf >= 0 ? 2 * (size_t)h->d.zds * plane : plane;
+  }
+  launch_interface_f64(h->hist + h->hn * hs, h->hist + h->hp * hs, h->hist + h->hpp * hs, h->iface_mac, tg, n, h->d,
+                       h->shape, h->g.omega_c, h->g.omega_f, st);
 }
 static void L_inject(dns_handle *h, int fbuf, int cbuf, cudaStream_t st) {
   if (is_f32(h))
@@ -1248,70 +1291,82 @@ extern "C" int dns_load_uniform(dns_handle *h, const char *dir, int cntr) {
   return refresh_flow(h, p.forcing == DNS_FORCING_CFR ? 0.0 : p.force_const);
 }
 
-// One coarse step on two streams.  The interface transfer of substep s
-// writes only the interface planes of the buffer whose other planes the fine
-// kernel of substep s writes, so the two run concurrently; the coarse kernel
-// and the extraction run beside the first fine substep.
-//   main:  coarse, extract, iface(1), [wait fine(s-1)] iface(s) ..., [wait inject] finalize
-//   aux:   [wait start] fine(1), [wait iface(s-1)] fine(s) ..., inject
-// (Measured on B200 with per-kernel device timestamps: the FP64 interface
-// transfer is bound by FP64 issue; moved with the extraction to a stream of
-// the greatest priority it ran beside the fine kernels but slowed them by as
-// much as it hid, 711 against 705 us per step, so it stays in order here.)
-// Schedule (compile-time): 0 one stream in order, 1 this schedule.
-#ifndef DNS_SCHED
-#define DNS_SCHED 1
-#endif
-static void issue_step_overlapped(dns_handle *h, DevLog *log_row, bool sample) {
+// One coarse step on two streams.  The fine substeps are taken in passes of two
+// (one read and one write of the fine state for both) or one.  A pass of two
+// needs the interface planes between its substeps before it starts; the
+// transfer of a pass's last substep writes only the interface planes of the
+// buffer whose other planes the pass writes, so the two may run concurrently.
+//   main:  coarse, extract, transfers (every plane between substeps, and the
+//          first pass's last substep), [wait pass i - 1] the last substep of
+//          pass i ..., [wait inject] finalize
+//   aux:   [wait start, or the transfers] pass 0, [wait transfer] pass 1 ..., inject
+// While profiling everything is issued on one stream, so that every launch can
+// be bracketed by its own pair of events.
+struct Pass {
+  int first, n, m;  // first substep, substeps, slot of the planes between them
+};
+static int plan_passes(const dns_handle *h, bool sample, Pass *out) {
+  int n = 0, m = 0;
+  for (int s = 1; s <= h->d.gr;) {
+    // the statistics of a sampled step are summed by the one-substep kernel
+    const bool two = pairs_on(h) && s < h->d.gr && !(sample && s == 1);
+    out[n++] = Pass{s, two ? 2 : 1, two ? m++ : -1};
+    s += two ? 2 : 1;
+  }
+  return n;
+}
+static void issue_step(dns_handle *h, DevLog *log_row, bool sample) {
   const Dims &d = h->d;
-  cudaStream_t S = h->stream, T = h->aux;
+  cudaStream_t S = h->stream, T = h->prof.on ? h->stream : h->aux;
+  auto signal = [&](cudaEvent_t e, cudaStream_t on, cudaStream_t waits) {
+    if (on == waits) return;
+    cudaEventRecord(e, on);
+    cudaStreamWaitEvent(waits, e, 0);
+  };
   const int nc = 1 - h->cur_c;
-  cudaEventRecord(h->ev_start, S);
-  cudaStreamWaitEvent(T, h->ev_start, 0);
-  L_coarse(h, h->cur_c, nc, sample, S);
+  Pass P[4];
+  const int np = plan_passes(h, sample, P);
+  signal(h->ev_start, S, T);
+  PROFILED(h, 0, L_coarse(h, h->cur_c, nc, sample, S));
   rotate_history(h);
-  L_extract(h, nc, h->hn, S);
+  PROFILED(h, 1, L_extract(h, nc, h->hn, S));
   int cur = h->cur_f;
-  for (int it = 1; it <= d.gr; it++) {
-    const int nf = 1 - cur;
-    if (it > 1) cudaStreamWaitEvent(T, h->ev_if[it - 2], 0);
-    L_fine(h, cur, nf, it == 1, it == d.gr, sample && it == 1, T);
-    cudaEventRecord(h->ev_fine[it - 1], T);
-    if (it > 1) cudaStreamWaitEvent(S, h->ev_fine[it - 2], 0);
-    L_iface(h, nf, it, S);
-    cudaEventRecord(h->ev_if[it - 1], S);
+  for (int i = 0; i < np; i++) {
+    const int nf = 1 - cur, last = P[i].first + P[i].n - 1;
+    auto transfer = [&] {
+      IfaceDest to[4];
+      int n = 0;
+      if (i == 0)
+        for (int q = 0; q < np; q++)
+          if (P[q].n == 2) to[n++] = IfaceDest{P[q].first, -1, P[q].m};
+      to[n++] = IfaceDest{last, nf, -1};
+      PROFILED(h, 3, L_iface(h, to, n, S));
+    };
+    auto fine = [&] {
+      if (P[i].n == 2)
+        PROFILED(h, 2, L_fine_pair(h, cur, nf, P[i].m, i == 0, i == np - 1, T));
+      else
+        PROFILED(h, 2, L_fine(h, cur, nf, i == 0, i == np - 1, sample && i == 0, T));
+    };
+    if (i == 0 && P[0].n == 2) {
+      transfer();
+      signal(h->ev_if[0], S, T);
+      fine();
+    } else {
+      fine();
+      transfer();
+      if (i + 1 < np) signal(h->ev_if[i], S, T);
+    }
+    // the next transfer overwrites interface planes of the buffer this pass reads
+    if (i + 1 < np) signal(h->ev_fine[i], T, S);
     cur = nf;
   }
-  L_inject(h, cur, nc, T);
-  cudaEventRecord(h->ev_inj, T);
-  cudaStreamWaitEvent(S, h->ev_inj, 0);
-  launch_finalize(h->state, log_row, h->partials, h->fin_counter, h->pl, d, h->shape, h->sp, S);
-  if (sample) launch_stats_finalize(h->stats_acc, h->partials, h->pl, d, h->shape, S);
+  PROFILED(h, 4, L_inject(h, cur, nc, T));
+  signal(h->ev_inj, T, S);
+  PROFILED(h, 5, launch_finalize(h->state, log_row, h->partials, h->fin_counter, h->pl, d, h->shape, h->sp,
+                                 P[0].n == 2, P[np - 1].n == 2, S));
+  if (sample) PROFILED(h, 6, launch_stats_finalize(h->stats_acc, h->partials, h->pl, d, h->shape, S));
   h->cur_f = cur;
-  h->cur_c = nc;
-}
-
-// The same step in stream order on one stream (used while profiling, so that
-// every launch can be bracketed by its own pair of events).
-static void issue_step(dns_handle *h, DevLog *log_row, bool sample) {
-  if (DNS_SCHED > 0 && !h->prof.on && d_gr_ok(h)) {
-    issue_step_overlapped(h, log_row, sample);
-    return;
-  }
-  const Dims &d = h->d;
-  const int nc = 1 - h->cur_c;
-  PROFILED(h, 0, L_coarse(h, h->cur_c, nc, sample, h->stream));
-  rotate_history(h);
-  PROFILED(h, 1, L_extract(h, nc, h->hn, h->stream));
-  for (int it = 1; it <= d.gr; it++) {
-    const int nf = 1 - h->cur_f;
-    PROFILED(h, 2, L_fine(h, h->cur_f, nf, it == 1, it == d.gr, sample && it == 1, h->stream));
-    PROFILED(h, 3, L_iface(h, nf, it, h->stream));
-    h->cur_f = nf;
-  }
-  PROFILED(h, 4, L_inject(h, h->cur_f, nc, h->stream));
-  PROFILED(h, 5, launch_finalize(h->state, log_row, h->partials, h->fin_counter, h->pl, d, h->shape, h->sp, h->stream));
-  if (sample) PROFILED(h, 6, launch_stats_finalize(h->stats_acc, h->partials, h->pl, d, h->shape, h->stream));
   h->cur_c = nc;
 }
 
@@ -1511,6 +1566,16 @@ extern "C" int dns_set_profiling(dns_handle *h, int on) {
       h->prof.cnt[c] = 0;
     }
   return DNS_OK;
+}
+
+extern "C" int dns_set_fine_pairs(dns_handle *h, int mode) {
+  if (!h || mode < -1 || mode > 1) return fail(DNS_EINVAL, "bad argument");
+  CUDA_TRY(cudaSetDevice(h->p.device));
+  const int before = h->pairs;
+  h->pairs = mode;
+  const int rc = pairs_on(h) ? ready_pairs(h) : DNS_OK;
+  if (rc) h->pairs = before;
+  return rc;
 }
 
 extern "C" int dns_kernel_times(dns_handle *h, double *ms, long *launches) {

@@ -48,6 +48,15 @@ struct Dims {
   int gr, nzs;
 };
 
+// Tiles of the kernels that take two fine substeps in one pass (pair_f64.cu):
+// ntx tiles along x and nly runs of ly rows along y, per block.
+struct PairGrid {
+  int ntx = 0, ly = 0, nly = 0;
+  int ns = 1;  // warps side by side along x (a tile is at most 32 ns - 2 nodes wide)
+  bool on() const { return ntx > 0; }
+  long blocks() const { return (long)ntx * nly; }  // per fine block
+};
+
 // Launch geometry shared by the kernels and the reductions.
 struct LaunchShape {
   int bx;          // threads per block along x
@@ -56,11 +65,26 @@ struct LaunchShape {
   int fgx, fgy;    // fine grid x/y blocks (z = 2 zds planes)
   int igx, igy;    // interface tile grid
   int jgx, jgy;    // injection / extraction grid (x, y) per wall
+  PairGrid pair;   // tiles of the passes that take two fine substeps
   long n_coarse_blocks() const { return (long)cgx * cgy; }  // per plane
   long n_fine_blocks() const { return (long)fgx * fgy; }    // per plane
 };
 
 LaunchShape make_shape(const Dims &d);
+
+constexpr int kPairMaxZds = 16;  // planes that fit the shared-memory ring
+PairGrid make_pair_grid(const Dims &d);  // off where zds > kPairMaxZds
+// whether they are faster than one substep at a time
+bool pairs_pay_f64(const Dims &d, const PairGrid &g);
+// raise the kernels' shared-memory limit on the current device (0, or -1)
+int prepare_pair_f64();
+// two substeps from src into dst; mid: the interface planes between them,
+// [2 walls][19][nyf][nxf]; part: per-block flow-rate pairs [2 g.blocks()] (last);
+// wpart: per-block wall-shear pairs [6][g.blocks()] (first)
+void launch_fine_pair_f64(const double *src, double *dst, const double *mid, const int8_t *wflag, const Dims &d,
+                          const PairGrid &g, double om, const DevState *st, double *part, double *wpart, bool first,
+                          bool last, cudaStream_t stream);
+
 
 // record a message for dns_last_error() on the calling thread (dns_api.cu)
 void set_last_error(const std::string &msg);
@@ -90,19 +114,27 @@ void launch_extract_f64(const double *fc, double *hist_n, const Dims &d, const L
 void launch_fine_f64(const double *src, double *dst, const int8_t *wflag, const Dims &d, const LaunchShape &s,
                      double om, const DevState *st, double *partials, const PartialLayout &pl, bool first,
                      bool last, bool stats, cudaStream_t stream);
-// two launches: macroscopic fields into mac[2 walls][4][nyf][nxf], then one
-// block per (tile, wall, population) into the interface planes of fdst
-void launch_interface_f64(const double *hn, const double *hp, const double *hpp, double *mac, double *fdst,
-                          const Dims &d, const LaunchShape &s, int substep, double omega_c, double omega_f,
+// The interface transfers of n substeps (at most 4), two launches: macroscopic
+// fields into mac[substep - 1][2 walls][4][nyf][nxf], then one block per (tile,
+// substep, wall, population) into the substep's planes
+struct IfaceTarget {
+  int substep;
+  void *out[2];   // plane of population 0 of the lower / upper wall
+  size_t stride;  // elements from one population's plane to the next
+};
+void launch_interface_f64(const double *hn, const double *hp, const double *hpp, double *mac, const IfaceTarget *tg,
+                          int n, const Dims &d, const LaunchShape &s, double omega_c, double omega_f,
                           cudaStream_t stream);
 // filtered: the FLTR transfer (ftcdtransfer_lesfltr.c) instead of ftcdtransfer.c
 void launch_inject_f64(const double *fsrc, double *cdst, const Dims &d, const LaunchShape &s, double omega_c,
                        double omega_f, double *partials, const PartialLayout &pl, bool filtered,
                        cudaStream_t stream);
-// counter: one device unsigned int, zero between launches (the kernel resets it)
+// counter: one device unsigned int, zero between launches (the kernel resets it);
+// pair_first / pair_last: the step's first / last fine pass took two substeps
+// (it left the wall-shear / flow-rate partials by its own tiles)
 void launch_finalize(DevState *st, DevLog *log_row, double *partials, unsigned int *counter,
                      const PartialLayout &pl, const Dims &d, const LaunchShape &s, const StepParams &sp,
-                     cudaStream_t stream);
+                     bool pair_first, bool pair_last, cudaStream_t stream);
 void launch_stats_finalize(double *acc, const double *partials, const PartialLayout &pl, const Dims &d,
                            const LaunchShape &s, cudaStream_t stream);
 // direct encalc2 reduction of the stored state into st (momentum, denst, force)

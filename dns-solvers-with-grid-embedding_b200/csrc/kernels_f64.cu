@@ -296,6 +296,14 @@ struct IfaceArgs {
   double h1, h2, h3, h4, fac;
 };
 
+// the substeps of one launch: blockIdx.z is ((substep * 2) + wall) * fields + field
+struct IfaceSet {
+  IfaceArgs a[4];
+  int mac[4];  // slot of the macroscopic fields
+  double *out[4][2];
+  size_t stride[4];
+};
+
 struct IfaceSmem {
   double V[PY][PX];
   double Dy[ITY + 1][PX];
@@ -390,21 +398,23 @@ __device__ __forceinline__ double iface_eval(const double (&cf)[16], int ii, int
   return val;
 }
 
-// Phase 1: macroscopic fields.  Block (tile, wall, field b < 4) writes field b
-// (rho, ux, uy, uz) at the tile's fine interface nodes into mac[wall][b][j][i].
+// Phase 1: macroscopic fields.  Block (tile, substep, wall, field b < 4) writes
+// field b (rho, ux, uy, uz) at the tile's fine interface nodes into
+// mac[substep][wall][b][j][i].
 template <int GR>
 __global__ void __launch_bounds__(TPX *TPY) interface_macro_kernel(const double *__restrict__ hn,
                                                                    const double *__restrict__ hp,
                                                                    const double *__restrict__ hpp,
-                                                                   double *__restrict__ mac, Dims d, IfaceArgs ia) {
+                                                                   double *__restrict__ mac, Dims d, IfaceSet is) {
   __shared__ IfaceSmem S;
   const int nx = d.nx, ny = d.ny, nxf = d.nxf, nyf = d.nyf;
-  const int w = blockIdx.z >> 2, b = blockIdx.z & 3;
+  const int sub = blockIdx.z >> 3, w = (blockIdx.z >> 2) & 1, b = blockIdx.z & 3;
+  const IfaceArgs &ia = is.a[sub];
   const int i0 = blockIdx.x * ITX, j0 = blockIdx.y * ITY;
   const int tx = threadIdx.x % TPX, ty = threadIdx.x / TPX;
   const size_t plane = (size_t)ny * nx, fplane = (size_t)nyf * nxf;
   iface_stage(S, hn, hp, hpp, ((size_t)w * 23 + b) * plane, i0, j0, nx, ny, ia);
-  double *o = mac + ((size_t)w * 4 + b) * fplane;
+  double *o = mac + ((size_t)(is.mac[sub] * 2 + w) * 4 + b) * fplane;
 #pragma unroll
   for (int q = 0; q < CPT; q++) {
     const int cx = tx + TPX * (q % (ITX / TPX)), cy = ty + TPY * (q / (ITX / TPX));
@@ -429,28 +439,27 @@ __global__ void __launch_bounds__(TPX *TPY) interface_macro_kernel(const double 
   }
 }
 
-// Phase 2: one population per block (tile, wall, a): feq(rho, u) of phase 1
-// plus omega_c / (GR omega_f) times the interpolated fneq, into the fine
-// block's interface plane.
+// Phase 2: one population per block (tile, substep, wall, a): feq(rho, u) of
+// phase 1 plus omega_c / (GR omega_f) times the interpolated fneq, into the
+// substep's interface plane of the wall's fine block.
 template <int GR>
 __global__ void __launch_bounds__(TPX *TPY) interface_pop_kernel(const double *__restrict__ hn,
                                                                  const double *__restrict__ hp,
                                                                  const double *__restrict__ hpp,
-                                                                 const double *__restrict__ mac,
-                                                                 double *__restrict__ fdst, Dims d, IfaceArgs ia) {
+                                                                 const double *__restrict__ mac, Dims d,
+                                                                 IfaceSet is) {
   __shared__ IfaceSmem S;
-  const int nx = d.nx, ny = d.ny, nxf = d.nxf, nyf = d.nyf, zds = d.zds;
-  const int w = blockIdx.z / 19, a = blockIdx.z % 19;
+  const int nx = d.nx, ny = d.ny, nxf = d.nxf, nyf = d.nyf;
+  const int sub = blockIdx.z / 38, w = (blockIdx.z / 19) & 1, a = blockIdx.z % 19;
+  const IfaceArgs &ia = is.a[sub];
   const int i0 = blockIdx.x * ITX, j0 = blockIdx.y * ITY;
   const int tx = threadIdx.x % TPX, ty = threadIdx.x / TPX;
   const size_t plane = (size_t)ny * nx, fplane = (size_t)nyf * nxf;
-  const int pf = w == 0 ? zds - 1 : zds;  // interface plane of the fine block
-  const size_t fstride = (size_t)2 * zds * fplane;
   iface_stage(S, hn, hp, hpp, ((size_t)w * 23 + 4 + a) * plane, i0, j0, nx, ny, ia);
   const int cls = a == 0 ? 0 : (a <= 6 ? 1 : 2);
   const double wa = cls == 0 ? 1. / 3. : (cls == 1 ? 1. / 18. : 1. / 36.);
-  const double *m = mac + (size_t)w * 4 * fplane;
-  double *out = fdst + (size_t)a * fstride + (size_t)pf * fplane;
+  const double *m = mac + (size_t)(is.mac[sub] * 2 + w) * 4 * fplane;
+  double *out = is.out[sub][w] + (size_t)a * is.stride[sub];
 #pragma unroll
   for (int q = 0; q < CPT; q++) {
     const int cx = tx + TPX * (q % (ITX / TPX)), cy = ty + TPY * (q / (ITX / TPX));
@@ -1001,6 +1010,7 @@ LaunchShape make_shape(const Dims &d) {
   s.igy = (d.ny + ITY - 1) / ITY;
   s.jgx = (d.nx + s.bx - 1) / s.bx;
   s.jgy = d.ny;
+  s.pair = make_pair_grid(d);
   return s;
 }
 
@@ -1008,11 +1018,12 @@ PartialLayout partial_layout(const Dims &d, const LaunchShape &s) {
   PartialLayout pl;
   const long nbc = s.n_coarse_blocks() * d.nzc, nbf = s.n_fine_blocks() * 2 * d.zds;
   const long nbi = (long)s.jgx * s.jgy * 2;
+  const long nbp = s.pair.blocks();  // a pass of two substeps: 2 nbp flow-rate pairs, 6 nbp wall pairs
   long o = 0;
   pl.coarse = o; o += nbc * 2;
-  pl.fine = o; o += nbf * 2;
+  pl.fine = o; o += (nbf > 2 * nbp ? nbf : 2 * nbp) * 2;
   pl.inject = o; o += nbi * 2;
-  pl.wall = o; o += nbf * 2;
+  pl.wall = o; o += (nbf > 6 * nbp ? nbf : 6 * nbp) * 2;
   pl.stats_c = o; o += nbc * kStatPart;
   pl.stats_f = o; o += nbf * kStatPart;
   const long gx = s.fgx > s.cgx ? s.fgx : s.cgx, gy = s.fgy > s.cgy ? s.fgy : s.cgy;
@@ -1053,28 +1064,34 @@ void launch_fine_f64(const double *src, double *dst, const int8_t *wflag, const 
 #undef FINE_CASE
 }
 
-void launch_interface_f64(const double *hn, const double *hp, const double *hpp, double *mac, double *fdst,
-                          const Dims &d, const LaunchShape &s, int substep, double omega_c, double omega_f,
+void launch_interface_f64(const double *hn, const double *hp, const double *hpp, double *mac, const IfaceTarget *tg,
+                          int n, const Dims &d, const LaunchShape &s, double omega_c, double omega_f,
                           cudaStream_t stream) {
-  // Hermite basis at tau = substep / GR, evaluated as the reference writes it
-  // (tinterpolate_hrmt.c:34); rescaling factor of ctfdtransfer_opt.c:101.
-  const double tmp = (((double)substep) / ((double)d.gr));
-  IfaceArgs ia;
-  ia.h1 = 2. * tmp * tmp * tmp - 3. * tmp * tmp + 1.;
-  ia.h2 = tmp * tmp * tmp - 2. * tmp * tmp + tmp;
-  ia.h3 = -2. * tmp * tmp * tmp + 3. * tmp * tmp;
-  ia.h4 = tmp * tmp * tmp - tmp * tmp;
-  ia.fac = omega_c / ((double)d.gr * omega_f);
-  dim3 gm(s.igx, s.igy, 2 * 4), gp(s.igx, s.igy, 2 * 19), block(TPX * TPY);
+  IfaceSet is{};
+  for (int q = 0; q < n; q++) {
+    // Hermite basis at tau = substep / GR, evaluated as the reference writes it
+    // (tinterpolate_hrmt.c:34); rescaling factor of ctfdtransfer_opt.c:101.
+    const double tmp = (((double)tg[q].substep) / ((double)d.gr));
+    IfaceArgs &ia = is.a[q];
+    ia.h1 = 2. * tmp * tmp * tmp - 3. * tmp * tmp + 1.;
+    ia.h2 = tmp * tmp * tmp - 2. * tmp * tmp + tmp;
+    ia.h3 = -2. * tmp * tmp * tmp + 3. * tmp * tmp;
+    ia.h4 = tmp * tmp * tmp - tmp * tmp;
+    ia.fac = omega_c / ((double)d.gr * omega_f);
+    is.mac[q] = tg[q].substep - 1;
+    for (int w = 0; w < 2; w++) is.out[q][w] = static_cast<double *>(tg[q].out[w]);
+    is.stride[q] = tg[q].stride;
+  }
+  dim3 gm(s.igx, s.igy, n * 2 * 4), gp(s.igx, s.igy, n * 2 * 19), block(TPX * TPY);
   if (d.gr == 2) {
-    interface_macro_kernel<2><<<gm, block, 0, stream>>>(hn, hp, hpp, mac, d, ia);
-    interface_pop_kernel<2><<<gp, block, 0, stream>>>(hn, hp, hpp, mac, fdst, d, ia);
+    interface_macro_kernel<2><<<gm, block, 0, stream>>>(hn, hp, hpp, mac, d, is);
+    interface_pop_kernel<2><<<gp, block, 0, stream>>>(hn, hp, hpp, mac, d, is);
   } else if (d.gr == 3) {
-    interface_macro_kernel<3><<<gm, block, 0, stream>>>(hn, hp, hpp, mac, d, ia);
-    interface_pop_kernel<3><<<gp, block, 0, stream>>>(hn, hp, hpp, mac, fdst, d, ia);
+    interface_macro_kernel<3><<<gm, block, 0, stream>>>(hn, hp, hpp, mac, d, is);
+    interface_pop_kernel<3><<<gp, block, 0, stream>>>(hn, hp, hpp, mac, d, is);
   } else {
-    interface_macro_kernel<4><<<gm, block, 0, stream>>>(hn, hp, hpp, mac, d, ia);
-    interface_pop_kernel<4><<<gp, block, 0, stream>>>(hn, hp, hpp, mac, fdst, d, ia);
+    interface_macro_kernel<4><<<gm, block, 0, stream>>>(hn, hp, hpp, mac, d, is);
+    interface_pop_kernel<4><<<gp, block, 0, stream>>>(hn, hp, hpp, mac, d, is);
   }
 }
 
@@ -1115,8 +1132,13 @@ static FinArgs fin_args(const PartialLayout &pl, const Dims &d, const LaunchShap
 
 void launch_finalize(DevState *st, DevLog *log_row, double *partials, unsigned int *counter,
                      const PartialLayout &pl, const Dims &d, const LaunchShape &s, const StepParams &sp,
-                     cudaStream_t stream) {
+                     bool pair_first, bool pair_last, cudaStream_t stream) {
   FinArgs a = fin_args(pl, d, s, sp);
+  if (pair_last) a.nf = 2 * s.pair.blocks();
+  if (pair_first) {
+    a.wn = s.pair.blocks();
+    for (int q = 0; q < 6; q++) a.wb[q] = q * a.wn;
+  }
   finalize2_kernel<<<kFin2Blocks, kFin2Threads, 0, stream>>>(st, log_row, partials + pl.coarse, partials + pl.fine,
                                                              partials + pl.inject, partials + pl.wall,
                                                              partials + pl.level2, counter, a);

@@ -143,6 +143,57 @@ __device__ __forceinline__ void collide_f64(double (&f)[19], double om, double G
 }
 
 
+// m / d from y = 1 / d correctly rounded: two residual corrections of m y with
+// fused multiply-adds.  The last one rounds correctly by Markstein's theorem
+// (IBM J. Res. Dev. 34, 1990): the value it corrects is a faithful rounding of
+// the quotient.  Not for non-finite operands.
+__device__ __forceinline__ double quotient_f64(double m, double d, double y) {
+  double q = m * y;
+  q = fma(fma(-q, d, m), y, q);
+  return fma(fma(-q, d, m), y, q);
+}
+
+// collide_f64 with opposite populations taken in pairs: e_b.u = -(e_a.u)
+// exactly, so 3 e.u and 4.5 (e.u)^2 are formed once for both, and one division
+// (the three velocities are quotients by the same density, and divisions of a
+// thread run one after another, 127 cycles each).  Every rounding is
+// collide_f64's; non-finite velocities are formed as it forms them.
+__device__ __forceinline__ void collide_pairs_f64(double (&f)[19], double om, double G, double &dens, double &u0,
+                                                  double &u1, double &u2) {
+  double mx, my, mz;
+  moments_f64(f, dens, mx, my, mz);
+  const double y = 1. / dens;
+  u0 = quotient_f64(mx, dens, y);
+  u1 = quotient_f64(my, dens, y);
+  u2 = quotient_f64(mz, dens, y);
+  double v = u0 * u0 + u1 * u1 + u2 * u2;
+  if (!(v <= 1e300)) {
+    u0 = mx / dens;
+    u1 = my / dens;
+    u2 = mz / dens;
+    v = u0 * u0 + u1 * u1 + u2 * u2;
+  }
+  const double t15v = 1.5 * v;
+  const Weighted wr = weighted_rho(dens);
+  const double q1 = (1. / 6.) * dens * G;
+  const double q2 = (1. / 12.) * dens * G;
+  f[0] = f[0] - om * (f[0] - wr.w0 * (1. - t15v));  // 1 + 3 0 + 4.5 0 0 = 1
+#pragma unroll
+  for (int a = 1; a < 19; a++) {
+    const int b = opp_of(a);
+    if (b < a) continue;
+    const double w = wclass_of(a) == 1 ? wr.w1 : wr.w2;
+    const double u = proj_f64(a, u0, u1, u2);
+    const double t3 = 3. * u, t45 = 4.5 * u * u;
+    const double ta = om * (f[a] - w * (1. + t3 + t45 - t15v));
+    const double tb = om * (f[b] - w * (1. - t3 + t45 - t15v));
+    const double q = wclass_of(a) == 1 ? q1 : q2;
+    const int ex = ex_of(a);
+    f[a] = ex == 0 ? f[a] - ta : (ex > 0 ? f[a] + (q - ta) : f[a] - (q + ta));
+    f[b] = ex == 0 ? f[b] - tb : (ex < 0 ? f[b] + (q - tb) : f[b] - (q + tb));
+  }
+}
+
 // ------------------------------------------------------------------ sampled statistics
 // Moments of a set of nodes' u, v, w, rho: count n, means m and sums of
 // squared deviations from the means q = (uu, vv, ww, uw, rr).  add() is

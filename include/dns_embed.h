@@ -224,6 +224,10 @@ int dns_plane_stats(dns_handle *h, double *out9xnz);
 #define DNS_NKERNEL 7
 int dns_set_profiling(dns_handle *h, int on);
 int dns_kernel_times(dns_handle *h, double *ms, long *launches);
+/* Fine substeps taken two at a time, in one pass over the fine state (zds <= 16
+   and an even GR xdv): -1 where the state is large enough to gain by it
+   (default), 0 never, 1 wherever possible.  The state is the same either way. */
+int dns_set_fine_pairs(dns_handle *h, int mode);
 
 /* ---- allocation-free reduction ------------------------------------------- */
 /* No counterpart in the reference.  For callers that cannot allocate device
