@@ -1481,75 +1481,29 @@ extern "C" int dns_stats(dns_handle *h, double *out, long *nsamples) {
 }
 
 // instantaneous plane statistics exactly as statistics.c:48-300 (two passes over
-// the exported state, same summation order)
+// the state, same summation order), on the device; the idle ping-pong buffers
+// hold the velocity fields (4 of the 19 populations' space, 8 of it in FP32)
 extern "C" int dns_plane_stats(dns_handle *h, double *out) {
   Range range("dns_plane_stats");
   if (!h || !out) return fail(DNS_EINVAL, "bad argument");
   CUDA_TRY(cudaSetDevice(h->p.device));
   const dns_geometry &g = h->g;
-  const int zdf = g.zdf, zdc = g.nzc, NZ = g.nz_profile;
-  std::vector<double> lv[3];
-  lv[0].resize(19ull * g.nzc * g.ny * g.nx);
-  lv[1].resize(19ull * g.zdf * g.nyf * g.nxf);
-  lv[2].resize(19ull * g.zdf * g.nyf * g.nxf);
-  int rc;
-  for (int l = 0; l < 3; l++)
-    if ((rc = export_level(h, l, lv[l].data()))) return rc;
-  static const int EX[19] = {0, 1, -1, 0, 0, 0, 0, 1, -1, -1, 1, 1, 1, -1, -1, 0, 0, 0, 0};
-  static const int EY[19] = {0, 0, 0, 1, -1, 0, 0, 1, 1, -1, -1, 0, 0, 0, 0, 1, 1, -1, -1};
-  static const int EZ[19] = {0, 0, 0, 0, 0, 1, -1, 0, 0, 0, 0, 1, -1, -1, 1, 1, -1, -1, 1};
-  double *U = out, *V = out + NZ, *W = out + 2 * NZ, *UT = out + 3 * NZ, *VT = out + 4 * NZ, *WT = out + 5 * NZ,
-         *RE = out + 6 * NZ, *DA = out + 7 * NZ, *DT = out + 8 * NZ;
+  const int zds = h->p.zds, npc = g.nzc - 4, NZ = g.nz_profile;
+  std::vector<double> fine((size_t)2 * zds * 9), coarse((size_t)npc * 9);
+  const int rc = plane_record_device(h->fc[h->cur_c], h->ff[h->cur_f], is_f32(h), h->fc[1 - h->cur_c],
+                                     h->ff[1 - h->cur_f], g, fine.data(), coarse.data(), h->stream);
+  if (rc) return rc;
   std::memset(out, 0, sizeof(double) * 9 * NZ);
-  struct Seg { int lvl, k0, k1, off, ex, ey, nz, d0, d1; } segs[3] = {
-      {1, 1, zdf, 0, g.nxf, g.nyf, zdf, 0, zdf},
-      {0, 2, zdc - 2, zdf - 2, g.nx, g.ny, zdc, zdf, zdf + zdc - 4},
-      {2, 0, zdf - 1, zdf + zdc - 4, g.nxf, g.nyf, zdf, zdf + zdc - 4, 2 * zdf + zdc - 4}};
-  for (int pass = 0; pass < 2; pass++)
-    for (const Seg &sg : segs) {
-      const double *a = lv[sg.lvl].data();
-      for (int i = 0; i < sg.ex; i++)
-        for (int j = 0; j < sg.ey; j++)
-          for (int k = sg.k0; k < sg.k1; k++) {
-            const double *f = a + (((size_t)i * sg.ey + j) * sg.nz + k) * 19;
-            double u = 0., v = 0., w = 0., dens = 0.;
-            for (int q = 0; q < 19; q++) {
-              dens += f[q];
-              u += (double)EX[q] * f[q];
-              v += (double)EY[q] * f[q];
-              w += (double)EZ[q] * f[q];
-            }
-            const int p = sg.off + k;
-            if (pass == 0) {
-              U[p] += (u / dens);
-              V[p] += (v / dens);
-              W[p] += (w / dens);
-              DA[p] += dens;
-            } else {
-              const double uf = (u / dens) - U[p], vf = (v / dens) - V[p], wf = (w / dens) - W[p],
-                           df = dens - DA[p];
-              UT[p] += uf * uf;
-              VT[p] += vf * vf;
-              WT[p] += wf * wf;
-              RE[p] += uf * wf;
-              DT[p] += df * df;
-            }
-          }
-      const double norm = (double)(sg.ex * sg.ey * 1 * 1);
-      for (int p = sg.d0; p < sg.d1; p++) {
-        if (pass == 0) {
-          U[p] /= norm; V[p] /= norm; W[p] /= norm; DA[p] /= norm;
-        } else {
-          UT[p] /= norm; VT[p] /= norm; WT[p] /= norm; RE[p] /= norm; DT[p] /= norm;
-        }
-      }
-    }
-  for (int p = 0; p < NZ; p++) {
-    UT[p] = std::sqrt(UT[p]);
-    VT[p] = std::sqrt(VT[p]);
-    WT[p] = std::sqrt(WT[p]);
-    DT[p] = std::sqrt(DT[p]);
+  auto put = [&](int p, const double *r) {  // UAVG VAVG WAVG UTIN VTIN WTIN REYS DAVG DTIN
+    const double v[9] = {r[0], r[1], r[2], std::sqrt(r[4]), std::sqrt(r[5]), std::sqrt(r[6]), r[7], r[3],
+                         std::sqrt(r[8])};
+    for (int c = 0; c < 9; c++) out[(size_t)c * NZ + p] = v[c];
+  };
+  for (int q = 0; q < zds; q++) {  // lower block k = q + 1, upper block k = q
+    put(q + 1, fine.data() + (size_t)q * 9);
+    put(g.zdf + g.nzc - 4 + q, fine.data() + (size_t)(zds + q) * 9);
   }
+  for (int q = 0; q < npc; q++) put(g.zdf + q, coarse.data() + (size_t)q * 9);
   return DNS_OK;
 }
 

@@ -192,6 +192,12 @@ int tke_budget_device(const dns_params &p, const dns_geometry &g, const double *
 size_t tke_workspace_bytes(const dns_geometry &g);
 int tke_budget_planar(const dns_params &p, const dns_geometry &g, const double *const q[3], double *prof,
                       double *ufl, double *vfl, cudaStream_t st, void *work = nullptr);
+// Plane statistics of the state (fc, ff) in the reference's summation order, one
+// row of 9 per plane: means of u, v, w, density, mean squares uu, vv, ww, uw, rr
+// about them.  fine: the 2 zds stored planes; coarse: planes 2..zdc-3.  qc, qf:
+// device scratch, (4 x nodes + 9) doubles a plane of each level.
+int plane_record_device(const void *fc, const void *ff, bool f32, double *qc, double *qf, const dns_geometry &g,
+                        double *fine, double *coarse, cudaStream_t st);
 // wall plane kw of a level in reference AoS order [nodes = nx ny][nz][19] to
 // (to_aos) or from the compact wall array [nodes][19]
 void launch_wall_plane(double *aos, double *wall, long long nodes, int nz, int kw, bool to_aos, cudaStream_t stream);

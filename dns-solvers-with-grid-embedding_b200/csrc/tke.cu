@@ -30,6 +30,7 @@
 
 #include "host.h"
 #include "kernels.h"
+#include "lattice.cuh"
 
 namespace dns {
 
@@ -98,44 +99,182 @@ __device__ __forceinline__ int profile_of(const TkeArgs &A, int l, int k) {
   return l == 1 ? k : (l == 0 ? A.zdf - 2 + k : A.zdf + A.zdc - 4 + k);
 }
 
-// plane means of the four fields of the profile planes k0.. of level L, each
-// summed in the reference's order (j outer, i inner: the plane's memory order)
-// and divided by the plane's node count (budget2D.c:178-241): the means, and
-// with them every fluctuation, are the reference's to the last bit.  The block
-// stages the plane through shared memory in coalesced chunks; threads 0..3
-// (u, v, w, den / 3) add each chunk in order.
-constexpr int kMeanChunk = 1024;
+// ------------------------------------------------------------ ordered sums
+// Sums of NF sequences of n values, each in sequence order (the reference's plane
+// loops: the results are its to the last bit).  The chain of n dependent adds
+// sets the time (8.3 cycles an add on B200: 0.57 ms for 131,072 nodes); everything
+// else is kept off it.  Warps 1.. form the values of a chunk in shared memory
+// while lanes 0..NF-1 of warp 0 add the previous one, each lane its own sequence,
+// sixteen values ahead in registers.  (Staged, waited for and added in turn by
+// the same warps, the same sums took 38 cycles an add.)
+// value(t, v): the NF values at position t.  Result in out[NF] (shared), visible
+// to every thread of the block on return; kSumThreads threads.
+constexpr int kSumChunk = 512, kSumThreads = 160;
+template <int NF>
+struct SumSmem {
+  // rows two banks apart: the adding lanes read the same position of NF rows
+  double buf[2][NF][kSumChunk + 2];
+};
 
-template <int L>
-__device__ __forceinline__ void mean_plane(const TkeArgs &A, int k, double (*buf)[kMeanChunk],
-                                           double *__restrict__ mean) {
-  const int nx = A.nx[L], ny = A.ny[L], nz = A.nz[L];
-  const size_t n = (size_t)nx * ny, field = (size_t)nz * n;
-  const double *q = A.q[L] + (size_t)k * n;
-  double s = 0.;
-  for (size_t base = 0; base < n; base += kMeanChunk) {
-    const int len = (int)(n - base < (size_t)kMeanChunk ? n - base : (size_t)kMeanChunk);
+template <int NF, class Value>
+__device__ __forceinline__ void ordered_sums(SumSmem<NF> &S, size_t n, Value value, double *out) {
+  static_assert(NF <= 32, "one lane a sequence");
+  constexpr int W = kSumThreads - 32, PER = kSumChunk / W;
+  const int t0 = (int)threadIdx.x - 32, lane = threadIdx.x & 31;
+  auto produce = [&](size_t base, int b) {
+    const int len = (int)(n - base < (size_t)kSumChunk ? n - base : (size_t)kSumChunk);
+    double v[PER][NF];
 #pragma unroll
-    for (int c = 0; c < 4; c++)
-      for (int t = threadIdx.x; t < len; t += blockDim.x) buf[c][t] = q[c * field + base + t];
-    __syncthreads();
-    if (threadIdx.x < 4) {
-      // unrolled so the shared-memory loads run ahead of the (ordered) adds
-#pragma unroll 16
-      for (int t = 0; t < len; t++) s += buf[threadIdx.x][t];
+    for (int r = 0; r < PER; r++)
+      if (t0 + r * W < len) value(base + t0 + r * W, v[r]);
+#pragma unroll
+    for (int r = 0; r < PER; r++)
+      if (t0 + r * W < len)
+#pragma unroll
+        for (int c = 0; c < NF; c++) S.buf[b][c][t0 + r * W] = v[r][c];
+  };
+  double s = 0.;
+  if (t0 >= 0) produce(0, 0);
+  __syncthreads();
+  int b = 0;
+  for (size_t base = 0; base < n; base += kSumChunk, b ^= 1) {
+    if (t0 >= 0) {
+      if (base + kSumChunk < n) produce(base + kSumChunk, b ^ 1);
+    } else if (lane < NF) {
+      const double *v = S.buf[b][lane];
+      const int len = (int)(n - base < (size_t)kSumChunk ? n - base : (size_t)kSumChunk);
+      if (len == kSumChunk) {
+        double2 x[8], y[8];
+        const double2 *w = reinterpret_cast<const double2 *>(v);
+#pragma unroll
+        for (int q = 0; q < 8; q++) x[q] = w[q];
+#pragma unroll 1
+        for (int t = 0; t < kSumChunk / 2; t += 16) {
+#pragma unroll
+          for (int q = 0; q < 8; q++) y[q] = w[t + 8 + q];
+#pragma unroll
+          for (int q = 0; q < 8; q++) {
+            s += x[q].x;
+            s += x[q].y;
+          }
+          if (t + 16 < kSumChunk / 2) {
+#pragma unroll
+            for (int q = 0; q < 8; q++) x[q] = w[t + 16 + q];
+          }
+#pragma unroll
+          for (int q = 0; q < 8; q++) {
+            s += y[q].x;
+            s += y[q].y;
+          }
+        }
+      } else {
+        for (int t = 0; t < len; t++) s += v[t];
+      }
     }
     __syncthreads();
   }
-  if (threadIdx.x < 4) mean[(size_t)profile_of(A, L, k) * 4 + threadIdx.x] = s / (double)(nx * ny);
+  if (t0 < 0 && lane < NF) out[lane] = s;
+  __syncthreads();
 }
 
+// plane means of u, v, w, den / 3, each plane summed in its memory order (j outer,
+// i inner: the reference's) and divided by its node count (budget2D.c:178-241);
 // one block per profile plane K
-__global__ void __launch_bounds__(kT) tke_mean_seq(TkeArgs A, double *__restrict__ mean) {
-  __shared__ double buf[4][kMeanChunk];
+__global__ void __launch_bounds__(kSumThreads) tke_mean_seq(TkeArgs A, double *__restrict__ mean) {
+  __shared__ SumSmem<4> S;
+  __shared__ double sum[4];
   const int K = blockIdx.x;
-  if (K < A.zdf) mean_plane<1>(A, K, buf, mean);
-  else if (K < A.zdf + A.zdc - 4) mean_plane<0>(A, K - A.zdf + 2, buf, mean);
-  else mean_plane<2>(A, K - (A.zdf + A.zdc - 4), buf, mean);
+  const int l = K < A.zdf ? 1 : (K < A.zdf + A.zdc - 4 ? 0 : 2);
+  const int k = l == 1 ? K : (l == 0 ? K - A.zdf + 2 : K - (A.zdf + A.zdc - 4));
+  const size_t n = (size_t)A.nx[l] * A.ny[l], field = (size_t)A.nz[l] * n;
+  const double *q = A.q[l] + (size_t)k * n;
+  ordered_sums<4>(S, n, [&](size_t t, double (&v)[4]) {
+#pragma unroll
+    for (int c = 0; c < 4; c++) v[c] = q[c * field + t];
+  }, sum);
+  if (threadIdx.x < 4) mean[(size_t)K * 4 + threadIdx.x] = sum[threadIdx.x] / (double)(A.nx[l] * A.ny[l]);
+}
+
+// ------------------------------------------------------------ plane-statistics record
+// statistics.c:48-300 on the device: per profile plane the means of u, v, w and
+// the density, then the mean squares of the deviations from them and of
+// u' w', each summed over the plane in the reference's order (i outer, j inner).
+// The fields first, per plane [c][plane][i][j], transposed through shared memory.
+template <class T>
+__device__ __forceinline__ double population(const T *p, int a);
+template <>
+__device__ __forceinline__ double population<double>(const double *p, int) {
+  return *p;
+}
+template <>
+__device__ __forceinline__ double population<float>(const float *p, int a) {  // as the exported state
+  const double w = a == 0 ? 1. / 3. : (a <= 6 ? 1. / 18. : 1. / 36.);
+  return w + (double)*p;
+}
+
+template <class T>
+__global__ void __launch_bounds__(256) record_fields(const T *__restrict__ soa, int nx, int ny, int P, int p0, int np,
+                                                     double *__restrict__ q) {
+  __shared__ double tile[4][32][33];
+  const int i0 = blockIdx.x * 32, j0 = blockIdx.y * 32, k = blockIdx.z;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const size_t plane = (size_t)ny * nx, stride = (size_t)P * plane;
+  const T *s = soa + (size_t)(p0 + k) * plane;
+  for (int r = ty; r < 32; r += 8)
+    if (i0 + tx < nx && j0 + r < ny) {
+      const T *f = s + (size_t)(j0 + r) * nx + i0 + tx;
+      double g[19];
+#pragma unroll
+      for (int a = 0; a < 19; a++) g[a] = population<T>(f + (size_t)a * stride, a);
+      double dens, mx, my, mz;
+      moments_f64(g, dens, mx, my, mz);
+      tile[0][r][tx] = mx / dens;
+      tile[1][r][tx] = my / dens;
+      tile[2][r][tx] = mz / dens;
+      tile[3][r][tx] = dens;
+    }
+  __syncthreads();
+  for (int r = ty; r < 32; r += 8)
+    if (i0 + r < nx && j0 + tx < ny)
+#pragma unroll
+      for (int c = 0; c < 4; c++) q[((size_t)c * np + k) * plane + (size_t)(i0 + r) * ny + j0 + tx] = tile[c][tx][r];
+}
+
+struct RecordLevel {
+  const double *q;  // [4][np][nodes]
+  double *out;      // [np][9]: means of u, v, w, density; mean squares uu, vv, ww, uw, rr
+  size_t nodes;     // per plane
+  int np;
+};
+// one block per plane, the fine level's first (they take longest)
+__global__ void __launch_bounds__(kSumThreads) record_sums(RecordLevel fine, RecordLevel coarse) {
+  __shared__ union {
+    SumSmem<4> a;
+    SumSmem<5> b;
+  } S;
+  __shared__ double mean[4], sum[5];
+  const bool f = (int)blockIdx.x < fine.np;
+  const RecordLevel &L = f ? fine : coarse;
+  const int k = f ? blockIdx.x : blockIdx.x - fine.np;
+  const size_t n = L.nodes, field = (size_t)L.np * n;
+  const double *q = L.q + (size_t)k * n;
+  const double norm = (double)n;
+  ordered_sums<4>(S.a, n, [&](size_t t, double (&v)[4]) {
+#pragma unroll
+    for (int c = 0; c < 4; c++) v[c] = q[c * field + t];
+  }, sum);
+  if (threadIdx.x < 4) mean[threadIdx.x] = L.out[(size_t)k * 9 + threadIdx.x] = sum[threadIdx.x] / norm;
+  __syncthreads();
+  ordered_sums<5>(S.b, n, [&](size_t t, double (&v)[5]) {
+    const double u = q[t] - mean[0], w = q[2 * field + t] - mean[2], vv = q[field + t] - mean[1],
+                 d = q[3 * field + t] - mean[3];
+    v[0] = u * u;
+    v[1] = vv * vv;
+    v[2] = w * w;
+    v[3] = u * w;
+    v[4] = d * d;
+  }, sum);
+  if (threadIdx.x < 5) L.out[(size_t)k * 9 + 4 + threadIdx.x] = sum[threadIdx.x] / norm;
 }
 
 // plane totals of W row partials in row order
@@ -560,7 +699,7 @@ int tke_budget_planar(const dns_params &p, const dns_geometry &g, const double *
   const int nyc = g.ny, nyf = g.nyf;
   cudaError_t e = cudaMemcpyAsync(dims, hdims.data(), NZ * sizeof(int), cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) {
-    tke_mean_seq<<<NZ, kT, 0, st>>>(A, mean);
+    tke_mean_seq<<<NZ, kSumThreads, 0, st>>>(A, mean);
     e = cudaGetLastError();
   }
   if (e == cudaSuccess) e = cudaMemsetAsync(part, 0, npart * 8, st);  // profile planes 0, NZ-1: no products
@@ -596,6 +735,30 @@ int tke_budget_planar(const dns_params &p, const dns_geometry &g, const double *
       }
   }
   return DNS_OK;
+}
+
+template <class T>
+static cudaError_t plane_record(const T *fc, const T *ff, double *qc, double *qf, const dns_geometry &g, double *fine,
+                                double *coarse, cudaStream_t st) {
+  const int zds = g.zdf - 1, npf = 2 * zds, npc = g.nzc - 4;
+  const size_t nf = (size_t)g.nxf * g.nyf, nc = (size_t)g.nx * g.ny;
+  const RecordLevel F{qf, qf + 4 * npf * nf, nf, npf}, C{qc, qc + 4 * npc * nc, nc, npc};
+  record_fields<T><<<dim3((g.nxf + 31) / 32, (g.nyf + 31) / 32, npf), 256, 0, st>>>(ff, g.nxf, g.nyf, npf, 0, npf, qf);
+  record_fields<T><<<dim3((g.nx + 31) / 32, (g.ny + 31) / 32, npc), 256, 0, st>>>(fc, g.nx, g.ny, g.nzc, 2, npc, qc);
+  record_sums<<<npf + npc, kSumThreads, 0, st>>>(F, C);
+  cudaError_t e = cudaGetLastError();
+  if (e == cudaSuccess) e = cudaMemcpyAsync(fine, F.out, (size_t)npf * 9 * 8, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(coarse, C.out, (size_t)npc * 9 * 8, cudaMemcpyDeviceToHost, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  return e;
+}
+
+int plane_record_device(const void *fc, const void *ff, bool f32, double *qc, double *qf, const dns_geometry &g,
+                        double *fine, double *coarse, cudaStream_t st) {
+  const cudaError_t e =
+      f32 ? plane_record(static_cast<const float *>(fc), static_cast<const float *>(ff), qc, qf, g, fine, coarse, st)
+          : plane_record(static_cast<const double *>(fc), static_cast<const double *>(ff), qc, qf, g, fine, coarse, st);
+  return e == cudaSuccess ? DNS_OK : fail_with(DNS_ECUDA, cudaGetErrorString(e));
 }
 
 int tke_budget_device(const dns_params &p, const dns_geometry &g, const double *const vel[3],
