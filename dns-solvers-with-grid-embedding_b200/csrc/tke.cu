@@ -53,14 +53,15 @@ static_assert(S_COUNT == kNS, "44 budget sums");
 struct TkeArgs {
   const double *q[3];  // planar fields per level (0 coarse, 1 lower fine, 2 upper fine)
   const double *mean;  // [NZ][4] plane means of u, v, w, den/3
-  double *part;        // [NZ][nymax][W] row partials
+  double *part;        // [NZ][nymax][W] partials of kRows rows each
   int nx[3], ny[3], nz[3];
   int gr, zdf, zdc, NZ, nymax;
   double coef;         // 1 / GR
 };
 
+// sum c of the block goes to out[to[c]]
 template <int N>
-__device__ __forceinline__ void block_sum(double (&v)[N], double *out) {
+__device__ __forceinline__ void block_sum(double (&v)[N], double *out, const unsigned char *to) {
   __shared__ double red[N][kT / 32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
@@ -75,9 +76,8 @@ __device__ __forceinline__ void block_sum(double (&v)[N], double *out) {
     double s = red[q][0];
 #pragma unroll
     for (int w = 1; w < kT / 32; w++) s += red[q][w];
-    out[q] = s;
+    out[to[q]] = s;
   }
-  __syncthreads();
 }
 
 // reference file layout vel[i][j][k][3], den[i][j][k] -> q[c][k][j][i]
@@ -105,8 +105,8 @@ __device__ __forceinline__ int profile_of(const TkeArgs &A, int l, int k) {
 // sets the time (8.3 cycles an add on B200: 0.57 ms for 131,072 nodes); everything
 // else is kept off it.  Warps 1.. form the values of a chunk in shared memory
 // while lanes 0..NF-1 of warp 0 add the previous one, each lane its own sequence,
-// sixteen values ahead in registers.  (Staged, waited for and added in turn by
-// the same warps, the same sums took 38 cycles an add.)
+// sixteen values ahead in registers: 0.58 ms for 131,072 nodes.  (Staged, waited
+// for and added in turn by the same warps: 38 cycles an add, 2.6 ms.)
 // value(t, v): the NF values at position t.  Result in out[NF] (shared), visible
 // to every thread of the block on return; kSumThreads threads.
 constexpr int kSumChunk = 512, kSumThreads = 160;
@@ -157,10 +157,8 @@ __device__ __forceinline__ void ordered_sums(SumSmem<NF> &S, size_t n, Value val
             s += x[q].x;
             s += x[q].y;
           }
-          if (t + 16 < kSumChunk / 2) {
 #pragma unroll
-            for (int q = 0; q < 8; q++) x[q] = w[t + 16 + q];
-          }
+          for (int q = 0; q < 8; q++) x[q] = w[(t + 16 + q) % (kSumChunk / 2)];  // the last ones are not used
 #pragma unroll
           for (int q = 0; q < 8; q++) {
             s += y[q].x;
@@ -335,21 +333,78 @@ __device__ __forceinline__ double ddz(const TkeArgs &A, int l, int c, int i, int
   return 0.5 * (fl(A, 2, c, i, j, k + 1) - fl(A, 2, c, i, j, k - 1));
 }
 
-// the 44 per-node terms of budget2D.c:448-624 (and the identical coarse and
-// upper bodies), summed over rows of the planes k0.. of level L (lower fine
-// 1..zdf-1, coarse 2..zdc-3, upper fine 0..zdf-2); grid (ny, planes)
-template <int L>
-__global__ void __launch_bounds__(kT) tke_budget_rows(TkeArgs A, int k0) {
-  constexpr int l = L;
-  const int j = blockIdx.x, k = k0 + blockIdx.y, K = profile_of(A, L, k);
-  double s[kNS];
+// The 44 per-node terms of budget2D.c:448-624 (and the identical coarse and
+// upper bodies), summed over kRows rows of plane k of level L (lower fine
+// 1..zdf-1, coarse 2..zdc-3, upper fine 0..zdf-2).  FP64 latency bounds it: two
+// kinds of block, one for the 28 products of the fluctuations alone, one for the
+// 16 with gradients, keep the sums of a thread in fewer registers (255 with
+// spills for all 44) and twice the warps on an SM; and as the block sums take as
+// many instructions as some five nodes of a thread, a block takes four rows.
+// 256x128x83: 633 us with one block a row and all sums, 503 us with four rows,
+// 393 / 320 / 304 us with two kinds of block at 3 / 4 / 5 of them on an SM.
+constexpr int kRows = 4;
+constexpr int kNV = 28, kNG = 16;
+__constant__ unsigned char c_val_sum[kNV] = {
+    S_UU, S_UV, S_UW, S_VV, S_VW, S_WW, S_DD, S_SKU, S_SKV, S_SKW, S_SKP, S_SKUW, S_SKUV, S_SKVW,
+    S_KUU, S_KUV, S_KUW, S_KUP, S_KUUW, S_KUVW, S_KUUV, S_UUW, S_VVW, S_WWW, S_UWW, S_PU, S_PV, S_PW};
+__constant__ unsigned char c_grad_sum[kNG] = {S_WX, S_WY, S_WZ, S_PAIUU, S_PAIVV, S_PAIWW, S_PAIUW, S_EPUU,
+                                              S_EPVV, S_EPWW, S_EPUW, S_USUW, S_VSVW, S_WSWW, S_WSUW, S_USWW};
+
+__device__ __forceinline__ void value_rows(const TkeArgs &A, int l, int k, int jb) {
+  const int K = profile_of(A, l, k), nx = A.nx[l], ny = A.ny[l];
+  const size_t n = (size_t)ny * nx, field = (size_t)A.nz[l] * n;
+  const double *q = A.q[l] + (size_t)k * n, *m = A.mean + (size_t)K * 4;
+  const double um = m[0], vm = m[1], wm = m[2], dm = m[3];
+  double s[kNV];
 #pragma unroll
-  for (int q = 0; q < kNS; q++) s[q] = 0.;
-  {
-    const int nx = A.nx[l], ny = A.ny[l];
+  for (int c = 0; c < kNV; c++) s[c] = 0.;
+  // the block's rows are one run of memory
+  const size_t lo = (size_t)jb * kRows * nx, hi = min(n, lo + (size_t)kRows * nx);
+  for (size_t t = lo + threadIdx.x; t < hi; t += blockDim.x) {
+    const double u = q[t] - um, v = q[field + t] - vm, w = q[2 * field + t] - wm, d = q[3 * field + t] - dm;
+    s[0] += u * u;
+    s[1] += u * v;
+    s[2] += u * w;
+    s[3] += v * v;
+    s[4] += v * w;
+    s[5] += w * w;
+    s[6] += d * d;
+    s[7] += u * u * u;
+    s[8] += v * v * v;
+    s[9] += w * w * w;
+    s[10] += d * d * d;
+    s[11] += u * u * u * w * w * w;
+    s[12] += u * u * u * v * v * v;
+    s[13] += v * v * v * w * w * w;
+    s[14] += u * u * u * u;
+    s[15] += v * v * v * v;
+    s[16] += w * w * w * w;
+    s[17] += d * d * d * d;
+    s[18] += u * u * u * u * w * w * w * w;
+    s[19] += v * v * v * v * w * w * w * w;
+    s[20] += u * u * u * u * v * v * v * v;
+    s[21] += u * u * w;
+    s[22] += v * v * w;
+    s[23] += w * w * w;
+    s[24] += u * w * w;
+    s[25] += u * d;
+    s[26] += v * d;
+    s[27] += w * d;
+  }
+  block_sum<kNV>(s, A.part + ((size_t)K * A.nymax + jb) * kNS, c_val_sum);
+}
+
+template <int L>
+__device__ __forceinline__ void gradient_rows(const TkeArgs &A, int k, int jb) {
+  constexpr int l = L;
+  const int K = profile_of(A, L, k), nx = A.nx[l], ny = A.ny[l];
+  const double cx = l == 0 ? A.coef : 1.;
+  const double davg = A.mean[K * 4 + 3];
+  double s[kNG];
+#pragma unroll
+  for (int c = 0; c < kNG; c++) s[c] = 0.;
+  for (int j = jb * kRows; j < min((jb + 1) * kRows, ny); j++) {
     const int jp = wrapn(j - 1, ny), jpp = wrapn(j - 2, ny), jn = wrapn(j + 1, ny), jnn = wrapn(j + 2, ny);
-    const double cx = l == 0 ? A.coef : 1.;
-    const double davg = A.mean[K * 4 + 3];
     for (int i = threadIdx.x; i < nx; i += blockDim.x) {
       const int ip = wrapn(i - 1, nx), ipp = wrapn(i - 2, nx), in = wrapn(i + 1, nx), inn = wrapn(i + 2, nx);
       const double u = fl(A, l, 0, i, j, k), v = fl(A, l, 1, i, j, k), w = fl(A, l, 2, i, j, k);
@@ -357,10 +412,11 @@ __global__ void __launch_bounds__(kT) tke_budget_rows(TkeArgs A, int k0) {
       double gx[3], gy[3], gz[3];
 #pragma unroll
       for (int c = 0; c < 3; c++) {
-        const double dx = (2. / 3.) * (fl(A, l, c, in, j, k) - fl(A, l, c, ip, j, k)) -
-                          (1. / 12.) * (fl(A, l, c, inn, j, k) - fl(A, l, c, ipp, j, k));
-        const double dy = (2. / 3.) * (fl(A, l, c, i, jn, k) - fl(A, l, c, i, jp, k)) -
-                          (1. / 12.) * (fl(A, l, c, i, jnn, k) - fl(A, l, c, i, jpp, k));
+        // along x and y the plane mean cancels
+        const double *qc = A.q[l] + ((size_t)c * A.nz[l] + k) * ny * nx, *qr = qc + (size_t)j * nx;
+        const double dx = (2. / 3.) * (qr[in] - qr[ip]) - (1. / 12.) * (qr[inn] - qr[ipp]);
+        const double dy = (2. / 3.) * (qc[(size_t)jn * nx + i] - qc[(size_t)jp * nx + i]) -
+                          (1. / 12.) * (qc[(size_t)jnn * nx + i] - qc[(size_t)jpp * nx + i]);
         gx[c] = l == 0 ? cx * dx : dx;
         gy[c] = l == 0 ? cx * dy : dy;
         gz[c] = ddz(A, l, c, i, j, k);
@@ -368,55 +424,47 @@ __global__ void __launch_bounds__(kT) tke_budget_rows(TkeArgs A, int k0) {
       const double dudx = gx[0], dvdx = gx[1], dwdx = gx[2];
       const double dudy = gy[0], dvdy = gy[1], dwdy = gy[2];
       const double dudz = gz[0], dvdz = gz[1], dwdz = gz[2];
-      s[S_UU] += u * u;
-      s[S_UV] += u * v;
-      s[S_UW] += u * w;
-      s[S_VV] += v * v;
-      s[S_VW] += v * w;
-      s[S_WW] += w * w;
-      s[S_SKU] += u * u * u;
-      s[S_SKV] += v * v * v;
-      s[S_SKW] += w * w * w;
-      s[S_SKP] += dfl * dfl * dfl;
-      s[S_SKUW] += u * u * u * w * w * w;
-      s[S_SKUV] += u * u * u * v * v * v;
-      s[S_SKVW] += v * v * v * w * w * w;
-      s[S_KUU] += u * u * u * u;
-      s[S_KUV] += v * v * v * v;
-      s[S_KUW] += w * w * w * w;
-      s[S_KUP] += dfl * dfl * dfl * dfl;
-      s[S_KUUW] += u * u * u * u * w * w * w * w;
-      s[S_KUVW] += v * v * v * v * w * w * w * w;
-      s[S_KUUV] += u * u * u * u * v * v * v * v;
-      s[S_DD] += dfl * dfl;
-      s[S_UUW] += u * u * w;
-      s[S_VVW] += v * v * w;
-      s[S_WWW] += w * w * w;
-      s[S_UWW] += u * w * w;
-      s[S_PU] += u * dfl;
-      s[S_PV] += v * dfl;
-      s[S_PW] += w * dfl;
       const double ox = (dwdy - dvdz), oy = (dudz - dwdx), oz = (dvdx - dudy);
-      s[S_WX] += ox * ox;
-      s[S_WY] += oy * oy;
-      s[S_WZ] += oz * oz;
-      s[S_PAIUU] += dfl * dudx;
-      s[S_PAIVV] += dfl * dvdy;
-      s[S_PAIWW] += dfl * dwdz;
-      s[S_PAIUW] += dfl * (dudz + dwdx);
-      s[S_USUW] += 0.5 * u * (dudz + dwdx);
-      s[S_VSVW] += 0.5 * v * (dvdz + dwdy);
-      s[S_WSWW] += 0.5 * w * (dwdz + dwdz);
-      s[S_WSUW] += 0.5 * w * (dudz + dwdx);
-      s[S_USWW] += 0.5 * u * (dwdz + dwdz);
-      s[S_EPUU] += dudx * (dudx + dudx) + dudy * (dudy + dvdx) + dudz * (dudz + dwdx);
-      s[S_EPVV] += dvdx * (dvdx + dudy) + dvdy * (dvdy + dvdy) + dvdz * (dvdz + dwdy);
-      s[S_EPWW] += dwdx * (dwdx + dudz) + dwdy * (dwdy + dvdz) + dwdz * (dwdz + dwdz);
-      s[S_EPUW] += dudx * (dwdx + dudz) + dudy * (dwdy + dvdz) + dudz * (dwdz + dwdz) + dwdx * (dudx + dudx) +
-                   dwdy * (dudy + dvdx) + dwdz * (dudz + dwdx);
+      s[0] += ox * ox;
+      s[1] += oy * oy;
+      s[2] += oz * oz;
+      s[3] += dfl * dudx;
+      s[4] += dfl * dvdy;
+      s[5] += dfl * dwdz;
+      s[6] += dfl * (dudz + dwdx);
+      s[7] += dudx * (dudx + dudx) + dudy * (dudy + dvdx) + dudz * (dudz + dwdx);
+      s[8] += dvdx * (dvdx + dudy) + dvdy * (dvdy + dvdy) + dvdz * (dvdz + dwdy);
+      s[9] += dwdx * (dwdx + dudz) + dwdy * (dwdy + dvdz) + dwdz * (dwdz + dwdz);
+      s[10] += dudx * (dwdx + dudz) + dudy * (dwdy + dvdz) + dudz * (dwdz + dwdz) + dwdx * (dudx + dudx) +
+               dwdy * (dudy + dvdx) + dwdz * (dudz + dwdx);
+      s[11] += 0.5 * u * (dudz + dwdx);
+      s[12] += 0.5 * v * (dvdz + dwdy);
+      s[13] += 0.5 * w * (dwdz + dwdz);
+      s[14] += 0.5 * w * (dudz + dwdx);
+      s[15] += 0.5 * u * (dwdz + dwdz);
     }
   }
-  block_sum<kNS>(s, A.part + ((size_t)K * A.nymax + j) * kNS);
+  block_sum<kNG>(s, A.part + ((size_t)K * A.nymax + jb) * kNS, c_grad_sum);
+}
+
+// both kinds of block of every level in one launch: the gradients, which take
+// longer, first, and of each the fine blocks' planes first
+__global__ void __launch_bounds__(kT, 5) tke_budget_rows(TkeArgs A) {
+  const int nf = (A.ny[1] + kRows - 1) / kRows, nc = (A.ny[0] + kRows - 1) / kRows, pf = A.zdf - 1, pc = A.zdc - 4;
+  const int half = 2 * nf * pf + nc * pc;
+  const bool grad = (int)blockIdx.x < half;
+  int b = grad ? blockIdx.x : blockIdx.x - half;
+  if (b < nf * pf) {
+    if (grad) gradient_rows<1>(A, 1 + b / nf, b % nf);
+    else value_rows(A, 1, 1 + b / nf, b % nf);
+  } else if ((b -= nf * pf) < nf * pf) {
+    if (grad) gradient_rows<2>(A, b / nf, b % nf);
+    else value_rows(A, 2, b / nf, b % nf);
+  } else {
+    b -= nf * pf;
+    if (grad) gradient_rows<0>(A, 2 + b / nc, b % nc);
+    else value_rows(A, 0, 2 + b / nc, b % nc);
+  }
 }
 
 // ------------------------------------------------------------ finalisation
@@ -655,7 +703,7 @@ int tke_validate(const dns_params &p) {
 
 size_t tke_workspace_bytes(const dns_geometry &g) {
   const size_t NZ = g.nz_profile;
-  return (NZ * g.nyf * kNS + NZ * 4 + NZ * kNS) * 8 + NZ * sizeof(int);
+  return (NZ * ((g.nyf + kRows - 1) / kRows) * kNS + NZ * 4 + NZ * kNS) * 8 + NZ * sizeof(int);
 }
 
 int tke_budget_planar(const dns_params &p, const dns_geometry &g, const double *const q[3], double *prof,
@@ -676,7 +724,7 @@ int tke_budget_planar(const dns_params &p, const dns_geometry &g, const double *
   A.zdf = g.zdf;
   A.zdc = g.nzc;
   A.NZ = g.nz_profile;
-  A.nymax = g.nyf;
+  A.nymax = (g.nyf + kRows - 1) / kRows;
   A.coef = (1. / ((double)g.gr));
   const int NZ = A.NZ;
   // budget2D.c:57-60, tauf the fine relaxation time
@@ -693,10 +741,10 @@ int tke_budget_planar(const dns_params &p, const dns_geometry &g, const double *
   int *dims = reinterpret_cast<int *>(buf + nbuf);
   double *part = buf, *mean = part + npart, *sums = mean + (size_t)NZ * 4;
   std::vector<int> hdims(NZ);
-  for (int K = 0; K < NZ; K++) hdims[K] = (K >= g.zdf && K < g.zdf + g.nzc - 4) ? g.ny : g.nyf;
+  const int nyc = (g.ny + kRows - 1) / kRows, nyf = (g.nyf + kRows - 1) / kRows;  // row blocks of a plane
+  for (int K = 0; K < NZ; K++) hdims[K] = (K >= g.zdf && K < g.zdf + g.nzc - 4) ? nyc : nyf;
   A.part = part;
   A.mean = mean;
-  const int nyc = g.ny, nyf = g.nyf;
   cudaError_t e = cudaMemcpyAsync(dims, hdims.data(), NZ * sizeof(int), cudaMemcpyHostToDevice, st);
   if (e == cudaSuccess) {
     tke_mean_seq<<<NZ, kSumThreads, 0, st>>>(A, mean);
@@ -704,9 +752,7 @@ int tke_budget_planar(const dns_params &p, const dns_geometry &g, const double *
   }
   if (e == cudaSuccess) e = cudaMemsetAsync(part, 0, npart * 8, st);  // profile planes 0, NZ-1: no products
   if (e == cudaSuccess) {
-    tke_budget_rows<1><<<dim3(nyf, g.zdf - 1), kT, 0, st>>>(A, 1);
-    tke_budget_rows<0><<<dim3(nyc, g.nzc - 4), kT, 0, st>>>(A, 2);
-    tke_budget_rows<2><<<dim3(nyf, g.zdf - 1), kT, 0, st>>>(A, 0);
+    tke_budget_rows<<<2 * (2 * nyf * (g.zdf - 1) + nyc * (g.nzc - 4)), kT, 0, st>>>(A);
     tke_sum_rows<<<NZ, 64, 0, st>>>(part, A.nymax, kNS, dims, sums);
     e = cudaGetLastError();
   }
