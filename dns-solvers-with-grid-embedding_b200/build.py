@@ -26,6 +26,7 @@ UNITS = {  # source -> extra flags
     "kernels_f64.cu": ["-fmad=false"],
     "pair_f64.cu": ["-fmad=false"],
     "kernels_f32.cu": [],
+    "pair_f32.cu": [],
     "batch_f32.cu": [],
     "dns_api.cu": [],
     "batch_api.cu": [],

@@ -315,7 +315,7 @@ static int refresh_flow(dns_batch *b, const Inst &I, const dns_params &q, const 
   if (cudaMallocAsync(&scratch, (size_t)flow_sums_pairs(d, shp) * 2 * 8, b->s) != cudaSuccess)
     return fail_with(DNS_ENOMEM, "flow-sum scratch");
   PartialLayout pl{};
-  const StepParams sp{g.omega_c, g.omega_f, q.ub, q.force_const, I.cfr, I.den_offset};
+  const StepParams sp{g.omega_c, g.omega_f, q.ub, q.force_const, I.cfr, I.fltr, I.den_offset};
   launch_flow_sums_f32(I.fc[cc], I.ff[cf], b->dstate + slot, scratch, pl, d, shp, sp, b->s);
   BTRY(cudaFreeAsync(scratch, b->s));
   return DNS_OK;

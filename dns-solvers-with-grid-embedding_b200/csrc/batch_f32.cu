@@ -345,12 +345,13 @@ __device__ __forceinline__ void iface_params_of(IfParams32 &P, const Inst &I, co
   P.hp = I.hist + (size_t)D.hn * hs;
   P.hpp = I.hist + (size_t)D.hp * hs;
   P.corner = I.corner + (size_t)(sub - 1) * 2 * 23 * I.ny * I.nx;  // substep sub's corner data
-  P.fdst = I.ff[D.cf ^ (sub & 1)];
+  const size_t fplane = (size_t)I.nyf * I.nxf;
+  for (int w = 0; w < 2; w++) P.out[w] = I.ff[D.cf ^ (sub & 1)] + (size_t)(I.zds - 1 + w) * fplane;
+  P.stride = (size_t)2 * I.zds * fplane;
   P.nx = I.nx;
   P.ny = I.ny;
   P.nxf = I.nxf;
   P.nyf = I.nyf;
-  P.zds = I.zds;
   P.an = tw.an;
   P.ap = tw.ap;
   P.app = tw.app;

@@ -36,7 +36,11 @@ int fail(int code, const std::string &msg) {
   } while (0)
 
 constexpr int kLogCap = 1024;
-constexpr int kXferChunks = 8;  // x runs per level transfer (state import / export)
+// x runs per level transfer (state import / export): up to 8 of at least 2 MB each,
+// below which a copy and its transpose are launches only (a 150 KB level: 9 us in
+// one run, 60 us in eight)
+constexpr int kXferChunks = 8;
+constexpr size_t kXferRun = 2 << 20;
 constexpr int kProfSteps = 256;  // steps per chunk while profiling (bounds the event pool)
 
 // CUDA-event timing of every launch (dns_set_profiling)
@@ -100,16 +104,19 @@ struct dns_handle {
 };
 
 // fine substeps are taken two at a time where the kernels allow it
-static bool pairs_built(const dns_handle *h) { return h->p.precision == DNS_FP64 && h->shape.pair.on(); }
+static bool pairs_pay(const dns_params &p, const Dims &d, const PairGrid &g) {
+  return p.precision == DNS_FP32 ? pairs_pay_f32(d, g) : pairs_pay_f64(d, g);
+}
 static bool pairs_on(const dns_handle *h) {
-  return pairs_built(h) && (h->pairs < 0 ? pairs_pay_f64(h->d, h->shape.pair) : h->pairs > 0);
+  return h->shape.pair.on() && (h->pairs < 0 ? pairs_pay(h->p, h->d, h->shape.pair) : h->pairs > 0);
 }
 
 // what the passes of two substeps need beyond the single ones
 static int ready_pairs(dns_handle *h) {
   if (h->iface_mid) return DNS_OK;
   const size_t bytes = (h->g.gr / 2) * 2ull * 19 * h->g.nyf * h->g.nxf * (h->p.precision == DNS_FP32 ? 4 : 8);
-  if (prepare_pair_f64()) return fail(DNS_ECUDA, "shared-memory limit of the two-substep kernels");
+  if (h->p.precision == DNS_FP32 ? prepare_pair_f32() : prepare_pair_f64())
+    return fail(DNS_ECUDA, "shared-memory limit of the two-substep kernels");
   if (cudaMalloc((void **)&h->iface_mid, bytes) != cudaSuccess)
     return fail(DNS_ENOMEM, "interface planes between two substeps");
   return DNS_OK;
@@ -279,12 +286,12 @@ extern "C" int dns_geometry_of(const dns_params *p, dns_geometry *g) {
   g->updates_per_step = (long long)p->xdv * p->ydv * p->zdv +
                         2LL * GR * ((long long)GR * p->xdv) * ((long long)GR * p->ydv) * p->zds;
   Dims d{g->nx, g->ny, g->nzc, g->nxf, g->nyf, g->zdf, p->zds, GR, g->nzs};
-  LaunchShape s = make_shape(d);
+  LaunchShape s = make_shape(d, p->precision == DNS_FP32);
   PartialLayout pl = partial_layout(d, s);
   const long long nc = 19LL * g->nzc * g->ny * g->nx, nf = 19LL * 2 * p->zds * g->nyf * g->nxf;
   const long long esz = p->precision == DNS_FP32 ? 4 : 8;  // bytes per stored population
   const long long mac = esz == 4 ? 2LL * 23 * g->ny * g->nx * 4 : 8LL * GR * g->nyf * g->nxf;  // elements of esz
-  const long long mid = esz == 8 && pairs_pay_f64(d, s.pair) ? (GR / 2) * 2LL * 19 * g->nyf * g->nxf : 0;
+  const long long mid = pairs_pay(*p, d, s.pair) ? (GR / 2) * 2LL * 19 * g->nyf * g->nxf : 0;
   g->device_bytes = esz * (2 * nc + 2 * nf + 3LL * 2 * 23 * g->ny * g->nx + mac + mid) +
                     8 * (pl.total + (long long)kStatRow * g->nz_profile + 2LL * 19 * g->nyf * g->nxf) +
                     (long long)g->nyf * g->nxf + (long long)kLogCap * sizeof(DevLog) + sizeof(DevState);
@@ -366,9 +373,9 @@ extern "C" int dns_create(const dns_params *p, dns_handle **out) {
   h->p = *p;
   h->g = g;
   h->d = Dims{g.nx, g.ny, g.nzc, g.nxf, g.nyf, g.zdf, p->zds, g.gr, g.nzs};
-  h->shape = make_shape(h->d);
+  h->shape = make_shape(h->d, p->precision == DNS_FP32);
   h->pl = partial_layout(h->d, h->shape);
-  h->sp = StepParams{g.omega_c, g.omega_f, p->ub, p->force_const, p->forcing == DNS_FORCING_CFR ? 1 : 0, 0.0};
+  h->sp = StepParams{g.omega_c, g.omega_f, p->ub, p->force_const, p->forcing == DNS_FORCING_CFR ? 1 : 0, p->fltr, 0.0};
   // the FP32 form's mass partials sum deviations from w: add the weight sum once
   if (p->precision == DNS_FP32) h->sp.den_offset = encalc2_weight_sum(h->d);
   const size_t esz = p->precision == DNS_FP32 ? 4 : 8;
@@ -395,6 +402,10 @@ extern "C" int dns_create(const dns_params *p, dns_handle **out) {
   // FP64: interface rho, u at fine nodes; FP32: corner values and derivatives (float4)
   const size_t mac_bytes = esz == 4 ? 2ull * 23 * g.ny * g.nx * 16 : 8ull * g.gr * g.nyf * g.nxf * esz;
   if ((rc = alloc((void **)&h->iface_mac, mac_bytes))) return rc;
+  if (p->fltr && (esz == 4 ? prepare_filter_f32() : prepare_filter_f64())) {
+    dns_destroy(h);
+    return fail(DNS_ECUDA, "shared-memory limit of the filtered injection");
+  }
   if (pairs_on(h) && (rc = ready_pairs(h))) {
     dns_destroy(h);
     return rc;
@@ -499,11 +510,17 @@ static int staging(dns_handle *h, int level, double **out) {
   return DNS_OK;
 }
 
+static int xfer_runs(const dns_handle *h, int level) {
+  if (!h->xfer_ok) return 1;
+  const size_t n = level_doubles(h->g, level) * 8 / kXferRun;
+  return n < 1 ? 1 : (n > kXferChunks ? kXferChunks : (int)n);
+}
+
 // One level of the post-stream state: device SoA (FP64, or FP32 deviations)
 // <-> reference AoS doubles on the host, through the device staging buffer:
 // the transpose and the wall plane (from / into wall_dev) are device kernels,
 // the host sees one copy of the whole level and one synchronisation.
-// A level moves in kXferChunks runs of x indices (contiguous on the AoS side):
+// A level moves in up to kXferChunks runs of x indices (contiguous on the AoS side):
 // the transpose of one run overlaps the host copy of another, the copies on
 // the second stream back to back.
 static void transpose_level(dns_handle *h, int level, double *stage, bool to_aos, int i0, int i1, cudaStream_t st) {
@@ -541,7 +558,7 @@ static int export_level(dns_handle *h, int level, double *out) {
   if (level > 0)
     launch_wall_plane(stage, h->wall_dev + (size_t)(level - 1) * g.nxf * g.nyf * 19, (long long)g.nxf * g.nyf,
                       g.zdf, level == 1 ? 0 : g.zdf - 1, true, h->stream);
-  const int C = h->xfer_ok ? kXferChunks : 1;
+  const int C = xfer_runs(h, level);
   cudaStream_t cs = C > 1 ? h->aux : h->stream;
   for (int c = 0; c < C; c++) {
     const int i0 = (int)((long long)nxl * c / C), i1 = (int)((long long)nxl * (c + 1) / C);
@@ -567,7 +584,7 @@ static int import_level(dns_handle *h, int level, const double *in) {
   if (rc) return rc;
   const int nxl = level == 0 ? g.nx : g.nxf;
   const size_t col = level_doubles(g, level) / (size_t)nxl;
-  const int C = h->xfer_ok ? kXferChunks : 1;
+  const int C = xfer_runs(h, level);
   cudaStream_t cs = C > 1 ? h->aux : h->stream;
   if (C > 1) {  // the copies follow whatever the handle's stream has queued
     CUDA_TRY(cudaEventRecord(h->ev_start, h->stream));
@@ -1141,9 +1158,14 @@ static void L_fine(dns_handle *h, int src, int dst, bool first, bool last, bool 
 }
 // Two substeps in one pass; m: slot of the interface planes between them
 static void L_fine_pair(dns_handle *h, int src, int dst, int m, bool first, bool last, cudaStream_t st) {
-  const double *mid = h->iface_mid + (size_t)m * 2 * 19 * h->d.nyf * h->d.nxf;
-  launch_fine_pair_f64(h->ff[src], h->ff[dst], mid, h->wflag, h->d, h->shape.pair, h->g.omega_f, h->state,
-                       h->partials + h->pl.fine, h->partials + h->pl.wall, first, last, st);
+  const size_t mid = (size_t)m * 2 * 19 * h->d.nyf * h->d.nxf;
+  double *part = h->partials + h->pl.fine, *wpart = h->partials + h->pl.wall;
+  if (is_f32(h))
+    launch_fine_pair_f32(F(h->ff[src]), F(h->ff[dst]), F(h->iface_mid) + mid, h->wflag, h->d, h->shape.pair,
+                         h->g.omega_f, h->state, part, wpart, first, last, st);
+  else
+    launch_fine_pair_f64(h->ff[src], h->ff[dst], h->iface_mid + mid, h->wflag, h->d, h->shape.pair, h->g.omega_f,
+                         h->state, part, wpart, first, last, st);
 }
 // Interface planes of substep it: those of the fine buffer fbuf, or (fbuf < 0)
 // slot m of the planes between two substeps of a pass
@@ -1151,23 +1173,24 @@ struct IfaceDest {
   int it, fbuf, m;
 };
 static void L_iface(dns_handle *h, const IfaceDest *to, int n, cudaStream_t st) {
-  const size_t hs = hslot_elems(h);
+  const size_t hs = hslot_elems(h), plane = (size_t)h->d.nyf * h->d.nxf;
+  IfaceTarget tg[4];
+  auto set = [&](auto *fine, auto *mid, IfaceTarget &t, const IfaceDest &d) {  // the form's own element type
+    t.substep = d.it;
+    for (int w = 0; w < 2; w++)
+      t.out[w] = fine ? fine + (size_t)(h->d.zds - 1 + w) * plane : mid + (size_t)(d.m * 2 + w) * 19 * plane;
+    t.stride = fine ? 2 * (size_t)h->d.zds * plane : plane;
+  };
   if (is_f32(h)) {
     float *H = F(h->hist);
-    for (int q = 0; q < n; q++)
-      launch_interface_f32(H + h->hn * hs, H + h->hp * hs, H + h->hpp * hs, F(h->iface_mac), F(h->ff[to[q].fbuf]),
-                           h->d, to[q].it, h->g.omega_c, h->g.omega_f, st);
+    for (int q = 0; q < n; q++) {
+      set(to[q].fbuf >= 0 ? F(h->ff[to[q].fbuf]) : nullptr, F(h->iface_mid), tg[q], to[q]);
+      launch_interface_f32(H + h->hn * hs, H + h->hp * hs, H + h->hpp * hs, F(h->iface_mac), tg[q], h->d,
+                           h->g.omega_c, h->g.omega_f, st);
+    }
     return;
   }
-  const size_t plane = (size_t)h->d.nyf * h->d.nxf;
-  IfaceTarget tg[4];
-  for (int q = 0; q < n; q++) {
-    tg[q].substep = to[q].it;
-    for (int w = 0; w < 2; w++)
-      tg[q].out[w] = to[q].fbuf >= 0 ? h->ff[to[q].fbuf] + (size_t)(h->d.zds - 1 + w) * plane
-                                     : h->iface_mid + (size_t)(to[q].m * 2 + w) * 19 * plane;
-    tg[q].stride = to[q].fbuf >= 0 ? 2 * (size_t)h->d.zds * plane : plane;
-  }
+  for (int q = 0; q < n; q++) set(to[q].fbuf >= 0 ? h->ff[to[q].fbuf] : nullptr, h->iface_mid, tg[q], to[q]);
   launch_interface_f64(h->hist + h->hn * hs, h->hist + h->hp * hs, h->hist + h->hpp * hs, h->iface_mac, tg, n, h->d,
                        h->shape, h->g.omega_c, h->g.omega_f, st);
 }

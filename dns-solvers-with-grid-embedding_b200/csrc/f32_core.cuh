@@ -374,30 +374,31 @@ __device__ __forceinline__ void fine_wall_f32(float (&f)[19], int i, int j, size
 struct IfParams32 {
   const float *hn, *hp, *hpp;  // history slots of levels n, p, pp: [2 walls][23][ny][nx]
   float4 *corner;              // corner data [2 walls][23][ny][nx]
-  float *fdst;                 // fine lattice receiving the interface planes
-  int nx, ny, nxf, nyf, zds;
+  float *out[2];               // plane of population 0 of the lower / upper wall
+  size_t stride;               // from one population's plane to the next
+  int nx, ny, nxf, nyf;
   float an, ap, app;           // Hermite-in-time weights of levels n, p, pp
   float fac;                   // omega_c / (GR omega_f): non-equilibrium rescaling
 };
 
 // launch parameters of one substep's transfer (substep s of GR: time s/GR)
-inline IfParams32 iface_params32(const float *hn, const float *hp, const float *hpp, float4 *corner, float *fdst,
-                                 const Dims &d, int substep, double omega_c, double omega_f) {
+inline IfParams32 iface_params32(const float *hn, const float *hp, const float *hpp, float4 *corner,
+                                 const IfaceTarget &tg, const Dims &d, double omega_c, double omega_f) {
   // value = h00 p + h10 (n - pp)/2 + h01 n + h11 (3n - 4p + pp)/2 (tinterpolate_hrmt.c:28-34),
   // gathered per level
-  const double t = (double)substep / (double)d.gr, t2 = t * t, t3 = t2 * t;
+  const double t = (double)tg.substep / (double)d.gr, t2 = t * t, t3 = t2 * t;
   const double h1 = 2. * t3 - 3. * t2 + 1., h2 = t3 - 2. * t2 + t, h3 = -2. * t3 + 3. * t2, h4 = t3 - t2;
   IfParams32 P;
   P.hn = hn;
   P.hp = hp;
   P.hpp = hpp;
   P.corner = corner;
-  P.fdst = fdst;
+  for (int w = 0; w < 2; w++) P.out[w] = static_cast<float *>(tg.out[w]);
+  P.stride = tg.stride;
   P.nx = d.nx;
   P.ny = d.ny;
   P.nxf = d.nxf;
   P.nyf = d.nyf;
-  P.zds = d.zds;
   P.an = (float)(0.5 * h2 + h3 + 1.5 * h4);
   P.ap = (float)(h1 - 2. * h4);
   P.app = (float)(-0.5 * h2 + 0.5 * h4);
@@ -689,9 +690,7 @@ __device__ __forceinline__ void iface_eval_tile32_gr2(IfEvalSmem<2> &S, const If
 #pragma unroll
     for (int h = 0; h < 2; h++)
       usq[r][h] = mac[1][r][h] * mac[1][r][h] + mac[2][r][h] * mac[2][r][h] + mac[3][r][h] * mac[3][r][h];
-  const size_t fplane = (size_t)P.nyf * P.nxf, fstride = (size_t)2 * P.zds * fplane;
-  const int pf = w == 0 ? P.zds - 1 : P.zds;
-  float *out = P.fdst + (size_t)pf * fplane;
+  float *out = P.out[w];
   for (int k = 4; k < nf; k++) {
     cp_async_wait<kEvalStages - 2>();
     __syncthreads();
@@ -700,7 +699,7 @@ __device__ __forceinline__ void iface_eval_tile32_gr2(IfEvalSmem<2> &S, const If
     float fv[NR][2];
     column(k, fv);
     const float ex = c_pop[a][0], ey = c_pop[a][1], ez = c_pop[a][2], wa = c_pop[a][3];
-    float *oa = out + (size_t)a * fstride;
+    float *oa = out + (size_t)a * P.stride;
 #pragma unroll
     for (int r = 0; r < NR; r++) {
       const int cy = cy0 + 2 * r;
@@ -773,9 +772,7 @@ __device__ __forceinline__ void iface_eval_tile32(IfEvalSmem<GR> &S, const IfPar
   float usq[NR];
 #pragma unroll
   for (int r = 0; r < NR; r++) usq[r] = mac[1][r] * mac[1][r] + mac[2][r] * mac[2][r] + mac[3][r] * mac[3][r];
-  const size_t fplane = (size_t)P.nyf * P.nxf, fstride = (size_t)2 * P.zds * fplane;
-  const int pf = w == 0 ? P.zds - 1 : P.zds;
-  float *out = P.fdst + (size_t)pf * fplane;
+  float *out = P.out[w];
   for (int k = 4; k < nf; k++) {
     cp_async_wait<kEvalStages - 2>();
     __syncthreads();
@@ -784,7 +781,7 @@ __device__ __forceinline__ void iface_eval_tile32(IfEvalSmem<GR> &S, const IfPar
     float fv[NR];
     if_column32<GR, NR>(S.C[k % kEvalStages], cx, ii, fy0, hx, fv);
     const float ex = c_pop[a][0], ey = c_pop[a][1], ez = c_pop[a][2], wa = c_pop[a][3];
-    float *oa = out + (size_t)a * fstride;
+    float *oa = out + (size_t)a * P.stride;
 #pragma unroll
     for (int r = 0; r < NR; r++) {
       const int fy = fy0 + 2 * r, cy = fy / GR, jj = fy - cy * GR;

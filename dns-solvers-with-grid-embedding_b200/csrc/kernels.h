@@ -65,22 +65,30 @@ struct LaunchShape {
   int fgx, fgy;    // fine grid x/y blocks (z = 2 zds planes)
   int igx, igy;    // interface tile grid
   int jgx, jgy;    // injection / extraction grid (x, y) per wall
-  PairGrid pair;   // tiles of the passes that take two fine substeps
+  int vgx;         // blocks of the filtered injection along x
+  PairGrid pair;   // tiles of the passes that take two fine substeps (of the precision asked for)
   long n_coarse_blocks() const { return (long)cgx * cgy; }  // per plane
   long n_fine_blocks() const { return (long)fgx * fgy; }    // per plane
 };
 
-LaunchShape make_shape(const Dims &d);
+LaunchShape make_shape(const Dims &d, bool f32 = false);
 
 constexpr int kPairMaxZds = 16;  // planes that fit the shared-memory ring
-PairGrid make_pair_grid(const Dims &d);  // off where zds > kPairMaxZds
+PairGrid make_pair_grid(const Dims &d);      // off where zds > kPairMaxZds
+PairGrid make_pair_grid_f32(const Dims &d);  // the FP32 form's tiles
+void pair_runs(const Dims &d, int per_sm, PairGrid &g);  // runs along y, per_sm blocks on an SM
 // whether they are faster than one substep at a time
 bool pairs_pay_f64(const Dims &d, const PairGrid &g);
+bool pairs_pay_f32(const Dims &d, const PairGrid &g);
 // raise the kernels' shared-memory limit on the current device (0, or -1)
 int prepare_pair_f64();
 // two substeps from src into dst; mid: the interface planes between them,
 // [2 walls][19][nyf][nxf]; part: per-block flow-rate pairs [2 g.blocks()] (last);
 // wpart: per-block wall-shear pairs [6][g.blocks()] (first)
+int prepare_pair_f32();
+void launch_fine_pair_f32(const float *src, float *dst, const float *mid, const int8_t *wflag, const Dims &d,
+                          const PairGrid &g, double om, const DevState *st, double *part, double *wpart, bool first,
+                          bool last, cudaStream_t stream);
 void launch_fine_pair_f64(const double *src, double *dst, const double *mid, const int8_t *wflag, const Dims &d,
                           const PairGrid &g, double om, const DevState *st, double *part, double *wpart, bool first,
                           bool last, cudaStream_t stream);
@@ -101,6 +109,7 @@ struct StepParams {
   double ub;        // bulk velocity (constant flow rate target)
   double gconst;    // constant body force
   int cfr;          // 1: force = ub - momentum
+  int fltr;         // the injection is the filtered one
   double den_offset;  // encalc2 weight sum added to the mass partials (FP32 form: they sum deviations)
 };
 
@@ -126,6 +135,9 @@ void launch_interface_f64(const double *hn, const double *hp, const double *hpp,
                           int n, const Dims &d, const LaunchShape &s, double omega_c, double omega_f,
                           cudaStream_t stream);
 // filtered: the FLTR transfer (ftcdtransfer_lesfltr.c) instead of ftcdtransfer.c
+// (its kernels' shared-memory limit is raised first, on the current device)
+int prepare_filter_f64();
+int prepare_filter_f32();
 void launch_inject_f64(const double *fsrc, double *cdst, const Dims &d, const LaunchShape &s, double omega_c,
                        double omega_f, double *partials, const PartialLayout &pl, bool filtered,
                        cudaStream_t stream);
@@ -218,8 +230,8 @@ void launch_fine_f32(const float *src, float *dst, const int8_t *wflag, const Di
                      double om, const DevState *st, double *partials, const PartialLayout &pl, bool first, bool last,
                      bool stats, cudaStream_t stream);
 // corner: scratch of 2 x 23 x ny x nx float4 (corner values and derivatives)
-void launch_interface_f32(const float *hn, const float *hp, const float *hpp, float *corner, float *fdst,
-                          const Dims &d, int substep, double omega_c, double omega_f, cudaStream_t stream);
+void launch_interface_f32(const float *hn, const float *hp, const float *hpp, float *corner, const IfaceTarget &tg,
+                          const Dims &d, double omega_c, double omega_f, cudaStream_t stream);
 void launch_inject_f32(const float *fsrc, float *cdst, const Dims &d, const LaunchShape &s, double omega_c,
                        double omega_f, double *partials, const PartialLayout &pl, bool filtered,
                        cudaStream_t stream);

@@ -3,6 +3,7 @@
 // interface evaluation) is in f32_core.cuh; layout, launch shapes and wall
 // rules follow kernels_f64.cu.
 #include "f32_core.cuh"
+#include "filter.cuh"
 #include "kernels.h"
 #include "lattice.cuh"
 #include "quad_f32.cuh"
@@ -315,28 +316,12 @@ __global__ void __launch_bounds__(kThreads) iface_eval_f32(IfParams32 P) {
 }
 
 // ------------------------------------------------------------------ injection
-template <bool FLT>
 __global__ void __launch_bounds__(kThreads) inject_f32(const float *__restrict__ fsrc, float *__restrict__ cdst, Dims d,
                                                       float fac, double *__restrict__ part) {
   const int nx = d.nx, ny = d.ny, nzc = d.nzc, gr = d.gr, zdf = d.zdf, zds = d.zds;
   const int ic = blockIdx.x * blockDim.x + threadIdx.x, jc = blockIdx.y, w = blockIdx.z;
   double acc[2] = {0., 0.};
-  if (FLT && ic < nx) {
-    float fo[19];
-    filtered_node_f32(fsrc, d.nxf, d.nyf, zds, zdf, gr, w, ic, jc, fac, fo);
-    const int kc = w == 0 ? 0 : nzc - 1;
-    const size_t cstride = (size_t)nzc * ny * nx;
-    float mom = 0.f, den = 0.f;
-#pragma unroll
-    for (int a = 0; a < 19; a++) {
-      cdst[(size_t)a * cstride + ((size_t)kc * ny + jc) * nx + ic] = fo[a];
-      den += fo[a];
-      if (ex_of(a) > 0) mom += fo[a];
-      if (ex_of(a) < 0) mom -= fo[a];
-    }
-    acc[0] = mom;
-    acc[1] = den;
-  } else if (!FLT && ic < nx) {
+  if (ic < nx) {
     const int ps = w == 0 ? (zdf - 1 - gr) - 1 : zds + gr;
     const size_t fstride = (size_t)2 * zds * d.nyf * d.nxf;
     float f[19];
@@ -359,6 +344,40 @@ __global__ void __launch_bounds__(kThreads) inject_f32(const float *__restrict__
   }
   const size_t blk = ((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
   block_reduce32<2>(acc, part + blk * 2);
+}
+
+// the filtered form in deviations (filter.cuh): f - w of the coarse node
+struct Filter32 {
+  using T = float;
+  using R = float;
+  static __device__ __forceinline__ void neq(const float (&f)[19], float (&n)[19], float (&m)[4]) {
+    const Mac32 c = macro_f32(f);
+    m[0] = c.drho;
+    m[1] = c.u0 * c.rho;
+    m[2] = c.u1 * c.rho;
+    m[3] = c.u2 * c.rho;
+#pragma unroll
+    for (int a = 0; a < 19; a++) n[a] = f[a] - deq_f32(a, c.drho, c.rho, c.u0, c.u1, c.u2, c.usq);
+  }
+  static __device__ __forceinline__ float add(float t, float wxy, float wz, float n) {
+    return t + (wxy * wz * (1.f / 64.f)) * n;
+  }
+  static __device__ __forceinline__ float result(int a, const float *m, float t, float fac) {
+    const float usq = m[1] * m[1] + m[2] * m[2] + m[3] * m[3];
+    float e = 0.f;
+#pragma unroll
+    for (int b = 0; b < 19; b++)
+      if (a == b) e = deq_f32(b, m[0], 1.f + m[0], m[1], m[2], m[3], usq);
+    return e + fac * t;
+  }
+};
+
+__global__ void __launch_bounds__(kFiltThreads) inject_filtered_f32(const float *__restrict__ fsrc,
+                                                                   float *__restrict__ cdst, Dims d, float fac,
+                                                                   double *__restrict__ part) {
+  extern __shared__ float filt_sm32[];
+  const size_t blk = ((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+  filtered_row<Filter32>(fsrc, cdst, d, blockIdx.x * kFiltV, blockIdx.y, blockIdx.z, fac, part + blk * 2, filt_sm32);
 }
 
 // ------------------------------------------------------------------ direct encalc2 sums
@@ -563,6 +582,13 @@ static bool quad_ok(const Dims &d, const LaunchShape &s) {
   return DNS_F32_QUAD_SINGLE && d.nx % 4 == 0 && s.bx == 4 * kQuadRow && s.jb == DNS_QUAD_JB;
 }
 
+int prepare_filter_f32() {
+  return cudaFuncSetAttribute(inject_filtered_f32, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)filter_smem<float>()) == cudaSuccess
+             ? 0
+             : -1;
+}
+
 void launch_coarse_f32(const float *src, float *dst, const Dims &d, const LaunchShape &s, double om,
                        const DevState *st, double *partials, const PartialLayout &pl, bool stats,
                        cudaStream_t stream) {
@@ -629,9 +655,9 @@ void launch_fine_f32(const float *src, float *dst, const int8_t *wflag, const Di
 #undef FINE32_CASE
 }
 
-void launch_interface_f32(const float *hn, const float *hp, const float *hpp, float *corner, float *fdst,
-                          const Dims &d, int substep, double omega_c, double omega_f, cudaStream_t stream) {
-  IfParams32 P = iface_params32(hn, hp, hpp, reinterpret_cast<float4 *>(corner), fdst, d, substep, omega_c, omega_f);
+void launch_interface_f32(const float *hn, const float *hp, const float *hpp, float *corner, const IfaceTarget &tg,
+                          const Dims &d, double omega_c, double omega_f, cudaStream_t stream) {
+  IfParams32 P = iface_params32(hn, hp, hpp, reinterpret_cast<float4 *>(corner), tg, d, omega_c, omega_f);
   dim3 gc((d.nx + CTX - 1) / CTX, (d.ny + CTY - 1) / CTY, 2 * kCornerFieldGroups);
   iface_corner_f32<<<gc, kThreads, 0, stream>>>(P);
 #define DNS_EVAL_LAUNCH(G)                                                                            \
@@ -650,9 +676,10 @@ void launch_inject_f32(const float *fsrc, float *cdst, const Dims &d, const Laun
   dim3 grid(s.jgx, s.jgy, 2), block(s.bx);
   const float fac = (float)(d.gr * (omega_f / omega_c));
   if (filtered)
-    inject_f32<true><<<grid, block, 0, stream>>>(fsrc, cdst, d, fac, partials + pl.inject);
+    inject_filtered_f32<<<dim3(s.vgx, d.ny, 2), kFiltThreads, filter_smem<float>(), stream>>>(fsrc, cdst, d, fac,
+                                                                                          partials + pl.inject);
   else
-    inject_f32<false><<<grid, block, 0, stream>>>(fsrc, cdst, d, fac, partials + pl.inject);
+    inject_f32<<<grid, block, 0, stream>>>(fsrc, cdst, d, fac, partials + pl.inject);
 }
 
 void launch_flow_sums_f32(const float *fc, const float *ff, DevState *st, double *partials, const PartialLayout &pl,

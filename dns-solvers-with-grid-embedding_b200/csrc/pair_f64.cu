@@ -44,6 +44,7 @@
 // for bit.  Built with -fmad=false.
 #include "kernels.h"
 #include "lattice.cuh"
+#include "pair_sync.cuh"
 
 namespace dns {
 
@@ -51,84 +52,11 @@ namespace {
 
 constexpr int kPairThreads = 32 * kPairMaxZds;
 
-// rows of population a that are live at a time, and where they start
-__host__ __device__ constexpr int ring_depth(int a) {
-  return a == 0 ? 0 : ey_of(a) < 0 ? ((a == 17 || a == 18) ? 2 : 1) : (ey_of(a) == 0 ? 2 : 3);
-}
-__host__ __device__ constexpr int ring_off(int a) {
-  int o = 0;
-  for (int b = 0; b < a; b++) o += ring_depth(b);
-  return o;
-}
-constexpr int kRing = ring_off(19);
-static_assert(kRing == 38, "live rows per plane");
-constexpr int kPad = 2;       // before and after the ring: pushes off its first and last row
-constexpr int kMaxRun = 256;  // rows of a run (the wall flags of a run are kept as one mask a row)
+constexpr int kPad = 2;  // before and after the ring: pushes off its first and last row
 
 // ring of zds - 1 planes, 19 rows of the interface plane, the next row of src
 size_t pair_smem(int zds, int ns) {
   return ((size_t)ns * 32 * ((zds - 1) * kRing + 19 + zds * 19) + 2 * kPad) * sizeof(double);
-}
-
-// Split barriers, one a plane: its warps and those of the planes beside it arrive
-// (only they push into its rows, and only it reads them), its warps wait for the
-// phase.  The waits are bounded: false after some 10 ms, which only a fault of
-// this file could cause (every warp makes the same arrivals).
-__device__ __forceinline__ void mb_init(unsigned long long *b, int count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"((unsigned)__cvta_generic_to_shared(b)), "r"(count)
-               : "memory");
-}
-// arrive at the barriers of planes q - 1, q, q + 1
-__device__ __forceinline__ void mb_arrive(unsigned long long *b, int lane, int q, int zds) {
-  __syncwarp();
-  const int n = q - 1 + lane;
-  if (lane < 3 && n >= 0 && n < zds)
-    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"((unsigned)__cvta_generic_to_shared(b + n))
-                 : "memory");
-}
-__device__ __forceinline__ bool mb_wait(unsigned long long *b, int parity) {
-  const unsigned a = (unsigned)__cvta_generic_to_shared(b);
-  for (int n = 0; n < (1 << 16); n++) {
-    unsigned ok;
-    asm volatile(
-        "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
-        : "=r"(ok)
-        : "r"(a), "r"(parity)
-        : "memory");
-    if (ok) return true;
-  }
-  return false;
-}
-
-// Bulk copies into a warp's rows: the warp's barrier completes when `bytes` have landed.
-__device__ __forceinline__ void mb_expect(unsigned long long *b, unsigned bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n" ::"r"((unsigned)__cvta_generic_to_shared(b)),
-               "r"(bytes)
-               : "memory");
-}
-__device__ __forceinline__ void bulk_copy(void *smem, const void *gmem, unsigned bytes, unsigned long long *b) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
-                   (unsigned)__cvta_generic_to_shared(smem)),
-               "l"(gmem), "r"(bytes), "r"((unsigned)__cvta_generic_to_shared(b))
-               : "memory");
-}
-
-// 8 bytes by the calling lane, its arrival at the barrier once they have landed
-__device__ __forceinline__ void lane_copy(void *smem, const void *gmem) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"((unsigned)__cvta_generic_to_shared(smem)), "l"(gmem)
-               : "memory");
-}
-__device__ __forceinline__ void lane_copies_arrive(unsigned long long *b) {
-  asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"((unsigned)__cvta_generic_to_shared(b))
-               : "memory");
-}
-
-// a thread-uniform base plus a 32-bit byte offset (population arrays are below 4 GB)
-__device__ __forceinline__ const double *at(const double *base, unsigned off) {
-  return reinterpret_cast<const double *>(reinterpret_cast<const char *>(base) + off);
-}
-__device__ __forceinline__ double *at(double *base, unsigned off) {
-  return reinterpret_cast<double *>(reinterpret_cast<char *>(base) + off);
 }
 
 // Keep the compiler from moving a node's collision into the branches that store
@@ -136,12 +64,6 @@ __device__ __forceinline__ double *at(double *base, unsigned off) {
 __device__ __forceinline__ void pin(double (&f)[19]) {
 #pragma unroll
   for (int a = 0; a < 19; a++) asm volatile("" : "+d"(f[a]));
-}
-
-// bits of the wall flags around a column: 0 own, 1 x + 1, 2 x - 1, 3 y + 1, 4 y - 1
-// (set: solid); the bit of the column population a heads for
-__host__ __device__ constexpr int dest_bit(int a) {
-  return ex_of(a) > 0 ? 2 : (ex_of(a) < 0 ? 4 : (ey_of(a) > 0 ? 8 : (ey_of(a) < 0 ? 16 : 1)));
 }
 
 // where tile i of n along a row of nx nodes starts: even, sizes at most two apart
@@ -160,7 +82,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   extern __shared__ double M[];
   constexpr int kTX = 32 * NS, kPlane = kRing * kTX;
   const int zds = d.zds, zdf = d.zdf, gr = d.gr, nx = d.nxf, ny = d.nyf;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // warp-uniform
   const bool upper = blockIdx.z != 0;
   // column c is node x0 + c (wrapped); tiles start at even nodes
   const int x0 = pair_x0(blockIdx.x, nx, g.ntx), cnt = pair_x0(blockIdx.x + 1, nx, g.ntx) - x0;
@@ -239,18 +161,17 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     }
     if (lane == 0) solid[r] = m;
   }
-  asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
+  fence_async_proxy();
   __syncthreads();
-  auto bits = [&](int t) {  // around column col of row t
-    const unsigned long long m = solid[t + 1];
-    return (int)((m >> col) & 1) | (int)(((m >> 1) >> col) & 1) << 1 | (int)(((m << 1) >> col) & 1) << 2 |
-           (int)((solid[t + 2] >> col) & 1) << 3 | (int)((solid[t] >> col) & 1) << 4;
-  };
   bool ok = true;
   double f[19], k0 = 0., p0 = 0.;  // population 0 of rows t and t - 1
   // the warp's columns of a row of 19 populations (stride apart) into rows
-  // `pitch` apart: lane a copies population a
+  // `pitch` apart: lane a copies population a.  (Every lane has collided the rows'
+  // old values; the fence puts the reads before the copies, which go by another
+  // way to shared memory.  Without it, and issued right behind the reads, copies
+  // overtook them.)
   auto copy = [&](double *row, int pitch, const double *from, size_t stride, unsigned long long *b) {
+    fence_async_proxy();
     __syncwarp();
     if (lane == 0) mb_expect(b, (unsigned)(19 * n1) * 8u);
     __syncwarp();
@@ -271,10 +192,10 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     if (t1 <= L + 1) ok = mb_wait(&staged[warp], t1 & 1) && ok;
 #pragma unroll
     for (int a = 0; a < 19; a++) f[a] = Sq[a * 32];
-    if (t1 <= L) stage(ahead);
     double dens, u0, u1, u2;
     collide_pairs_f64(f, om, Gf, dens, u0, u1, u2);
     pin(f);
+    if (t1 <= L) stage(ahead);
     if ((MODE & 2) && own && t1 >= 1 && t1 <= L) {
       if (wall_sum_plane) wacc[0] += u0;
       if (wall_rho_plane) wacc[1] += dens;
@@ -310,7 +231,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
             for (int a = 1; a < 19; a++)
               if (ez_of(a) == c) to(a)[slot(a, ey_of(a)) + ex_of(a)] = f[a];
         if (wall) {
-          const int sb = bits(t);
+          const int sb = solid_bits(solid, t, col);
 #pragma unroll
           for (int a = 1; a < 19; a++) {
             if (ez_of(a) == 0 || (ez_of(a) > 0) != upper) continue;
@@ -329,11 +250,11 @@ __global__ void __launch_bounds__(kPairThreads, 1)
       h[a] = Mr[iface ? a * kTX : ring_off(a) * kTX + (ring_depth(a) == 1 ? 0 : (ring_depth(a) == 2 ? r2p : r3p))];
     h[0] = iface ? Mr[0] : p0;
     mb_arrive(taken, lane, q, zds);
-    if (iface && t >= 1 && t <= L)  // the interface row that substep 2 takes next (row t)
-      copy(Mq - lane, kTX, mid + ((size_t)(upper ? 19 : 0) * ny + y) * nx, plane, &middle[warp]);
     double dens, u0, u1, u2;
     collide_pairs_f64(h, om, Gf, dens, u0, u1, u2);
     pin(h);
+    if (iface && t >= 1 && t <= L)  // the interface row that substep 2 takes next (row t)
+      copy(Mq - lane, kTX, mid + ((size_t)(upper ? 19 : 0) * ny + y) * nx, plane, &middle[warp]);
     if (t >= 2 && own) {
       if ((MODE & 1) && unit) {
         acc[0] += dens * u0 + dens * Gf;
@@ -358,7 +279,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
             for (int a = 0; a < 19; a++)
               if (ez_of(a) == c) *at(dst + (size_t)a * pstride, o + off(a) + offz(a)) = h[a];
         if (wall) {
-          const int sb = bits(t - 1);
+          const int sb = solid_bits(solid, t - 1, col);
 #pragma unroll
           for (int a = 0; a < 19; a++) {
             if (ez_of(a) == 0 || (ez_of(a) > 0) != upper) continue;
@@ -416,29 +337,34 @@ __global__ void __launch_bounds__(kPairThreads, 1)
 
 }  // namespace
 
-// Tiles of a fine block: two warps side by side where two segments of planes
-// fit the ring and the row is longer than one.  Runs along y: the number that
-// gives the shortest schedule of one block per SM (rows of a run, the two
-// redundant rows and about two rows' worth of start and end, times the waves).
-PairGrid make_pair_grid(const Dims &d) {
-  PairGrid g;
-  // 32-bit byte offsets in a population; rows of 16-byte multiples
-  if (d.zds > kPairMaxZds || 2LL * d.zds * d.nyf * d.nxf >= (1LL << 29) || d.nxf % 2) return g;
+// The number of runs along y that gives the shortest schedule: rows of a run, the
+// two redundant rows and about two rows' worth of start and end, times the waves.
+void pair_runs(const Dims &d, int per_sm, PairGrid &g) {
   constexpr int kSm = 148;
-  g.ns = (2 * d.zds <= kPairMaxZds && d.nxf > 30) ? 2 : 1;
-  const int w = 32 * g.ns - 2;
-  g.ntx = (d.nxf + w - 1) / w;
   long best = -1;
   for (int n = 1; n <= d.nyf && n <= 1024; n++) {
     const int ly = (d.nyf + n - 1) / n, nly = (d.nyf + ly - 1) / ly;
     if (ly > kMaxRun) continue;
-    const long waves = (2L * g.ntx * nly + kSm - 1) / kSm, cost = waves * (ly + 4);
+    const long waves = (2L * g.ntx * nly + kSm * per_sm - 1) / (kSm * per_sm), cost = waves * (ly + 4);
     if (best < 0 || cost < best) {
       best = cost;
       g.ly = ly;
       g.nly = nly;
     }
   }
+  if (best < 0) g.ntx = 0;  // more rows than runs can hold
+}
+
+// Tiles of a fine block: two warps side by side where two segments of planes
+// fit the ring and the row is longer than one.
+PairGrid make_pair_grid(const Dims &d) {
+  PairGrid g;
+  // 32-bit byte offsets in a population; rows of 16-byte multiples
+  if (d.zds > kPairMaxZds || 2LL * d.zds * d.nyf * d.nxf >= (1LL << 29) || d.nxf % 2) return g;
+  g.ns = (2 * d.zds <= kPairMaxZds && d.nxf > 30) ? 2 : 1;
+  const int w = 32 * g.ns - 2;
+  g.ntx = (d.nxf + w - 1) / w;
+  pair_runs(d, 1, g);
   return g;
 }
 

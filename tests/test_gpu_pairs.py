@@ -8,7 +8,7 @@ import numpy as np
 import pytest
 
 from conftest import gpu_available
-from test_gpu_parity import assert_state, pair
+from test_gpu_parity import assert_state, pair, params_for
 
 pytestmark = [pytest.mark.gpu, pytest.mark.skipif(not gpu_available(), reason="no CUDA device")]
 
@@ -48,6 +48,27 @@ def test_pairs_match_oracle(pkg, port, grid, mode):
     np.testing.assert_allclose(la[:, 5:8], lb[:, 4:7], rtol=1e-9, atol=1e-14)
 
 
+@pytest.mark.parametrize("grid", GRIDS, ids=lambda g: "x".join(str(v) for v in g[:5]))
+def test_fp32_pairs_match_single_substeps(pkg, grid):
+    """The FP32 form's pairs against its single substeps: the same arithmetic in
+    another grouping, five steps: within 5e-7 (a collision rounds a deviation of at
+    most 0.03 a few times, some 1e-8; at most 20 substeps)."""
+    m = macros(*grid)
+    p = params_for(pkg, m, "const")
+    p.precision = pkg.FP32
+    out = []
+    for mode in (0, 1):
+        with pkg.Channel(p) as ch:
+            ch.set_fine_pairs(mode)
+            ch.init_seeded(42, 0.05, 0.005)
+            log = ch.step(5)
+            out.append(([ch.export_state(lvl) for lvl in range(3)], log))
+    for a, b in zip(out[0][0], out[1][0]):
+        np.testing.assert_allclose(a, b, rtol=0, atol=5e-7)
+    # momentum, mass, flow rate: sums of the states compared above
+    np.testing.assert_allclose(out[0][1][:, 2:5], out[1][1][:, 2:5], rtol=1e-5)
+
+
 def test_pairs_and_single_substeps_mix(pkg, port):
     """Sampled steps (their first substep alone) between steps in pairs, ratio 4
     with the filtered transfer: the oracle's state, whatever was on before."""
@@ -61,3 +82,19 @@ def test_pairs_and_single_substeps_mix(pkg, port):
         assert_state(ch, p, exact=True)
     _, n = ch.stats()
     assert n == 4  # steps 0, 3, 6, 9
+
+
+def test_pairs_match_single_substeps_on_a_full_gpu(pkg):
+    """Sixteen planes, every SM busy, 40 substeps: the same bits as the single
+    substeps (rows that copies bring in while others are read)."""
+    kw = dict(xdv=128, ydv=128, zdv=51, zds=16, gratio=2, Rebs=3000.0, ub=0.0866034, CFL=0.1, pattern="RSLIP",
+              gyplussize=24, wyplussize=8, forcing=pkg.FORCING_CONST, force_const=1e-5)
+    states = []
+    for mode in (0, 1):
+        with pkg.Channel(pkg.make_params(**kw)) as ch:
+            ch.set_fine_pairs(mode)
+            ch.init_seeded(42, 0.05, 0.005)
+            ch.step(20)
+            states.append([ch.export_state(lvl) for lvl in range(3)])
+    for a, b in zip(*states):
+        np.testing.assert_array_equal(a, b)
