@@ -322,6 +322,16 @@ std::vector<int8_t> dns::wall_flags(const dns_params &p, const dns_geometry &g) 
 }
 
 // ---------------------------------------------------------------- lifecycle
+// The handle's stream.  From ratio 3 on, where a step waits for its interface
+// transfers most often, it goes before the fine substeps' stream (60 steps of the
+// 96x48x55 channel of ratio 4: 55.2 -> 52.2 ms, 75x45x31 of ratio 3: 11.6 -> 11.4
+// ms; ratio 2 gained nothing, 64x64x27 lost 2%).
+static cudaError_t create_stream(dns_handle *h) {
+  int low = 0, high = 0;
+  cudaDeviceGetStreamPriorityRange(&low, &high);
+  return cudaStreamCreateWithPriority(&h->stream, cudaStreamNonBlocking, h->d.gr >= 3 ? high : low);
+}
+
 extern "C" void dns_destroy(dns_handle *h) {
   if (!h) return;
   cudaSetDevice(h->p.device);
@@ -418,13 +428,13 @@ extern "C" int dns_create(const dns_params *p, dns_handle **out) {
     dns_destroy(h);
     return fail(DNS_ENOMEM, "cudaMallocHost failed");
   }
-  if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) {
+  int prio_low = 0, prio_high = 0;
+  cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high);
+  if (create_stream(h) != cudaSuccess) {
     dns_destroy(h);
     return fail(DNS_ECUDA, "cudaStreamCreate failed");
   }
   h->own_stream = true;
-  int prio_low = 0, prio_high = 0;
-  cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high);
   bool ev_ok = cudaStreamCreateWithPriority(&h->aux, cudaStreamNonBlocking, prio_low) == cudaSuccess;
   cudaEvent_t *evs[] = {&h->ev_start, &h->ev_inj, &h->ev_fine[0], &h->ev_fine[1], &h->ev_fine[2],
                         &h->ev_fine[3], &h->ev_if[0], &h->ev_if[1], &h->ev_if[2], &h->ev_if[3]};
@@ -461,7 +471,7 @@ extern "C" int dns_set_stream(dns_handle *h, void *cuda_stream) {
     h->stream = (cudaStream_t)cuda_stream;
     h->own_stream = false;
   } else if (!h->own_stream) {
-    CUDA_TRY(cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking));
+    CUDA_TRY(create_stream(h));
     h->own_stream = true;
   }
   return DNS_OK;
