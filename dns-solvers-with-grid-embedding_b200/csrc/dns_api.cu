@@ -36,6 +36,17 @@ int fail(int code, const std::string &msg) {
   } while (0)
 
 constexpr int kLogCap = 1024;
+// Steps recorded as one graph.  Issued one by one a step is 11 to 15 launches and
+// 8 or more event calls: 43 to 62 us of host time, and gaps of 2 to 5 us on the
+// device wherever one stream waits for the other.  us a step, one by one and from a
+// graph, FP64: 12x6x9 46.2 / 31.2, 64x64x27 89 / 84, 96x48x55 at ratio 4 476 / 470,
+// 256x128x83 556 / 545; FP32: 64x64x27 66 / 59, 131x77x45 171 / 158, 256x128x83
+// 345..362 / 345; host time below 1 us.  kGraphSteps is the period of the buffers
+// (two) and the history ring (three).  Recording takes 0.5 to 0.8 ms, as much as 8
+// (smallest channel) to 30 groups save, so a group is recorded when it is due for the
+// kGraphAfter-th time; kStepGraphs bounds them: the six states that steps can start a
+// group from, sampled or not.
+constexpr int kGraphSteps = 6, kStepGraphs = 12, kGraphAfter = 8;
 // x runs per level transfer (state import / export): up to 8 of at least 2 MB each,
 // below which a copy and its transpose are launches only (a 150 KB level: 9 us in
 // one run, 60 us in eight)
@@ -54,6 +65,15 @@ struct Profiler {
 };
 
 }  // namespace
+
+// kGraphSteps coarse steps recorded once and issued by one launch.  The ping-pong
+// buffers and the history ring are back where they were after that many steps.
+struct StepGraph {
+  int cur_c, cur_f, hn;  // buffers and ring slot of the first step
+  bool sample;           // every step sampled, or none
+  int seen;              // times such a group was due
+  cudaGraphExec_t exec;
+};
 
 struct dns_handle {
   dns_params p{};
@@ -80,7 +100,7 @@ struct dns_handle {
   size_t tke_ws_bytes = 0;
   double *tke_wall = nullptr;          // planar fields of the two wall planes [2][4][nyf][nxf]
   long tke_wall_gen = -1;              // wall_gen they were made from
-  unsigned int *fin_counter = nullptr; // finalize's block counter
+  unsigned int *fin_counter = nullptr; // finalize's block counter and log row
   cudaStream_t aux = nullptr;          // fine substeps and injection (lowest priority)
   cudaEvent_t ev_start = nullptr, ev_inj = nullptr, ev_fine[4] = {}, ev_if[4] = {};
   cudaEvent_t ev_xfer[kXferChunks] = {};  // one per x run of a level transfer
@@ -100,8 +120,13 @@ struct dns_handle {
   bool wall_host_stale = false;
   long wall_gen = 0;                     // bumped whenever the wall planes change
   double *stage = nullptr;               // FP32 form: one level in reference AoS doubles (allocated on first use)
+  StepGraph graphs[kStepGraphs];         // groups of steps issued by one graph launch
+  int ngraphs = 0;
+  bool graphs_ok = true;
   Profiler prof;
 };
+
+static void drop_graphs(dns_handle *h);
 
 // fine substeps are taken two at a time where the kernels allow it
 static bool pairs_pay(const dns_params &p, const Dims &d, const PairGrid &g) {
@@ -340,6 +365,7 @@ extern "C" void dns_destroy(dns_handle *h) {
     cudaFree(h->fc[q]);
     cudaFree(h->ff[q]);
   }
+  drop_graphs(h);
   cudaFree(h->hist);
   cudaFree(h->wflag);
   cudaFree(h->partials);
@@ -1348,9 +1374,9 @@ static int plan_passes(const dns_handle *h, bool sample, Pass *out) {
   }
   return n;
 }
-static void issue_step(dns_handle *h, DevLog *log_row, bool sample) {
+static void issue_step(dns_handle *h, cudaStream_t S, bool sample) {
   const Dims &d = h->d;
-  cudaStream_t S = h->stream, T = h->prof.on ? h->stream : h->aux;
+  cudaStream_t T = h->prof.on ? S : h->aux;
   auto signal = [&](cudaEvent_t e, cudaStream_t on, cudaStream_t waits) {
     if (on == waits) return;
     cudaEventRecord(e, on);
@@ -1396,11 +1422,68 @@ static void issue_step(dns_handle *h, DevLog *log_row, bool sample) {
   }
   PROFILED(h, 4, L_inject(h, cur, nc, T));
   signal(h->ev_inj, T, S);
-  PROFILED(h, 5, launch_finalize(h->state, log_row, h->partials, h->fin_counter, h->pl, d, h->shape, h->sp,
+  PROFILED(h, 5, launch_finalize(h->state, h->dlog, h->partials, h->fin_counter, h->pl, d, h->shape, h->sp,
                                  P[0].n == 2, P[np - 1].n == 2, S));
   if (sample) PROFILED(h, 6, launch_stats_finalize(h->stats_acc, h->partials, h->pl, d, h->shape, S));
   h->cur_f = cur;
   h->cur_c = nc;
+}
+
+static void drop_graphs(dns_handle *h) {
+  for (int q = 0; q < h->ngraphs; q++)
+    if (h->graphs[q].exec) cudaGraphExecDestroy(h->graphs[q].exec);
+  h->ngraphs = 0;
+}
+
+// The FP32 form's quad kernels at ratio 3 and 4 on larger channels go one by one:
+// us a step, one by one and from a graph, 96x64x40 at ratio 3 (2.9 M node updates)
+// 170.6 / 172.6, 96x64x50 at ratio 4 (8.2 M) 298 / 303, but 75x45x31 (1.4 M) 147 / 123
+// and 48x32x30 at ratio 4 (1.6 M) 116 / 115.
+static bool groups_pay(const dns_handle *h) {
+  const Dims &d = h->d;
+  const long updates = 2L * d.gr * d.zds * d.nyf * d.nxf + (long)d.nx * d.ny * d.nzc;
+  return !(is_f32(h) && d.gr >= 3 && d.nx % 4 == 0 && updates > 2500000L);
+}
+
+// Records kGraphSteps steps on a stream of its own (the handle's may be one that
+// cannot be recorded), the main chain above the fine substeps: with both alike the
+// coarse level starts behind a fine substep (FP32 256x128x83: 354 us a step, not 345).
+// A failure leaves the handle to issue its steps one by one.
+static cudaGraphExec_t record_steps(dns_handle *h, bool sample) {
+  int low = 0, high = 0;
+  cudaStream_t S = nullptr;
+  cudaGraph_t graph = nullptr;
+  cudaGraphExec_t exec = nullptr;
+  if (cudaDeviceGetStreamPriorityRange(&low, &high) == cudaSuccess &&
+      cudaStreamCreateWithPriority(&S, cudaStreamNonBlocking, high) == cudaSuccess &&
+      cudaStreamBeginCapture(S, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+    for (int q = 0; q < kGraphSteps; q++) issue_step(h, S, sample);
+    if (cudaStreamEndCapture(S, &graph) != cudaSuccess ||
+        cudaGraphInstantiate(&exec, graph, cudaGraphInstantiateFlagUseNodePriority) != cudaSuccess)
+      exec = nullptr;
+  }
+  if (graph) cudaGraphDestroy(graph);
+  if (S) cudaStreamDestroy(S);
+  if (!exec) {
+    h->graphs_ok = false;
+    cudaGetLastError();
+  }
+  return exec;
+}
+
+// The graph of the next kGraphSteps steps, or null where they are issued one by one
+static cudaGraphExec_t step_graph(dns_handle *h, bool sample) {
+  if (!h->graphs_ok || !groups_pay(h)) return nullptr;
+  int q = 0;
+  for (; q < h->ngraphs; q++) {
+    const StepGraph &G = h->graphs[q];
+    if (G.cur_c == h->cur_c && G.cur_f == h->cur_f && G.hn == h->hn && G.sample == sample) break;
+  }
+  if (q == kStepGraphs) return nullptr;
+  if (q == h->ngraphs) h->graphs[h->ngraphs++] = StepGraph{h->cur_c, h->cur_f, h->hn, sample, 0, nullptr};
+  StepGraph &G = h->graphs[q];
+  if (!G.exec && ++G.seen >= kGraphAfter) G.exec = record_steps(h, sample);
+  return G.exec;
 }
 
 extern "C" int dns_step(dns_handle *h, long ncoarse, dns_step_log *log) {
@@ -1413,10 +1496,18 @@ extern "C" int dns_step(dns_handle *h, long ncoarse, dns_step_log *log) {
   while (done < ncoarse) {
     const long n = std::min<long>(h->prof.on ? kProfSteps : kLogCap, ncoarse - done);
     const long ss0 = h->ss;
-    for (long q = 0; q < n; q++) {
-      const bool sample = h->sample_every > 0 && (h->ss % h->sample_every) == 0;
-      issue_step(h, h->dlog + q, sample);
-      h->ss++;
+    auto sampled = [&](long s) { return h->sample_every > 0 && s % h->sample_every == 0; };
+    CUDA_TRY(cudaMemsetAsync(h->fin_counter + 1, 0, 4, h->stream));
+    for (long q = 0; q < n;) {
+      const bool sample = sampled(h->ss);
+      long run = 1;  // steps from here on that are sampled like this one
+      while (run < kGraphSteps && q + run < n && sampled(h->ss + run) == sample) run++;
+      cudaGraphExec_t G = run == kGraphSteps && !h->prof.on ? step_graph(h, sample) : nullptr;
+      if (G) CUDA_TRY(cudaGraphLaunch(G, h->stream));
+      else
+        for (long r = 0; r < run; r++) issue_step(h, h->stream, sample);
+      q += run;
+      h->ss += run;
     }
     CUDA_TRY(cudaGetLastError());
     CUDA_TRY(cudaMemcpyAsync(h->hlog, h->dlog, n * sizeof(DevLog), cudaMemcpyDeviceToHost, h->stream));
@@ -1559,6 +1650,7 @@ extern "C" int dns_set_fine_pairs(dns_handle *h, int mode) {
   if (!h || mode < -1 || mode > 1) return fail(DNS_EINVAL, "bad argument");
   CUDA_TRY(cudaSetDevice(h->p.device));
   const int before = h->pairs;
+  drop_graphs(h);
   h->pairs = mode;
   const int rc = pairs_on(h) ? ready_pairs(h) : DNS_OK;
   if (rc) h->pairs = before;

@@ -144,7 +144,9 @@ void launch_inject_f64(const double *fsrc, double *cdst, const Dims &d, const La
 // counter: one device unsigned int, zero between launches (the kernel resets it);
 // pair_first / pair_last: the step's first / last fine pass took two substeps
 // (it left the wall-shear / flow-rate partials by its own tiles)
-void launch_finalize(DevState *st, DevLog *log_row, double *partials, unsigned int *counter,
+// log: the rows of a group of steps; counter[1] is the next row, counter[0] the
+// kernel's block count (0 between launches)
+void launch_finalize(DevState *st, DevLog *log, double *partials, unsigned int *counter,
                      const PartialLayout &pl, const Dims &d, const LaunchShape &s, const StepParams &sp,
                      bool pair_first, bool pair_last, cudaStream_t stream);
 void launch_stats_finalize(double *acc, const double *partials, const PartialLayout &pl, const Dims &d,

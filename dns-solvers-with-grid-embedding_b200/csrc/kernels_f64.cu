@@ -681,7 +681,8 @@ __global__ void __launch_bounds__(kFinThreads) finalize_kernel(DevState *st, Dev
 // kFin2Blocks blocks, each a fixed slice, the last of which to finish sums the
 // others' rows.  Fixed orders, no waiting.  It is latency: the chain of one block's
 // loads, sums and the log row, whose quotients lanes form side by side (a division
-// is 127 cycles, a thread's run one after another).  Small channel (64x64x27):
+// is 127 cycles, a thread's run one after another).  The log row's index is counter[1],
+// advanced here, so that a step's launches are the same from step to step.  Small channel (64x64x27):
 // 7.0 us with 64 blocks, 18 block sums in each and one thread's log row.
 constexpr int kFin2Blocks = 64, kFin2Threads = 256, kFin2Comp = 18, kFin1Threads = 1024;
 constexpr long kFin1Pairs = 4096;
@@ -768,6 +769,7 @@ __global__ void __launch_bounds__(NT) finalize2_kernel(DevState *st, DevLog *lg,
   // lanes 0..4: flow rate, lower and upper wall shear, momentum, mass
   const double *S = sh, *U = sh + 6;  // (U, D) pairs per plane: lower k=1,2,3, upper zdf-2,-3,-4
   const double m0 = st->momentum, d0 = st->denst, f0 = st->force;
+  const unsigned int at_row = counter[1];
   double num, den, fac = 1.;
   if (lane == 0) {
     num = m0 * a.flow_scale;
@@ -800,7 +802,8 @@ __global__ void __launch_bounds__(NT) finalize2_kernel(DevState *st, DevLog *lg,
     r.stdown = stdown;
     r.stress = 0.5 * (stup + stdown);
     r.pgrad = f0 * a.pgrad_scale;
-    *lg = r;
+    lg[at_row] = r;
+    counter[1] = at_row + 1;
     st->momentum = mom;
     st->denst = mass;
     st->force = a.cfr ? a.ub - mom : a.gconst;
@@ -1132,7 +1135,7 @@ static FinArgs fin_args(const PartialLayout &pl, const Dims &d, const LaunchShap
   return a;
 }
 
-void launch_finalize(DevState *st, DevLog *log_row, double *partials, unsigned int *counter,
+void launch_finalize(DevState *st, DevLog *log, double *partials, unsigned int *counter,
                      const PartialLayout &pl, const Dims &d, const LaunchShape &s, const StepParams &sp,
                      bool pair_first, bool pair_last, cudaStream_t stream) {
   FinArgs a = fin_args(pl, d, s, sp);
@@ -1143,10 +1146,10 @@ void launch_finalize(DevState *st, DevLog *log_row, double *partials, unsigned i
   }
   double *pc = partials + pl.coarse, *pf = partials + pl.fine, *pi = partials + pl.inject, *pw = partials + pl.wall;
   if (a.nc + a.nf + a.ni + 6 * a.wn <= kFin1Pairs)
-    finalize2_kernel<kFin1Threads><<<1, kFin1Threads, 0, stream>>>(st, log_row, pc, pf, pi, pw, partials + pl.level2,
+    finalize2_kernel<kFin1Threads><<<1, kFin1Threads, 0, stream>>>(st, log, pc, pf, pi, pw, partials + pl.level2,
                                                                    counter, a);
   else
-    finalize2_kernel<kFin2Threads><<<kFin2Blocks, kFin2Threads, 0, stream>>>(st, log_row, pc, pf, pi, pw,
+    finalize2_kernel<kFin2Threads><<<kFin2Blocks, kFin2Threads, 0, stream>>>(st, log, pc, pf, pi, pw,
                                                                              partials + pl.level2, counter, a);
 }
 
