@@ -676,26 +676,14 @@ static int export_history(dns_handle *h, double *out) {
   return DNS_OK;
 }
 
+// The idle fine buffer, every plane of which the next step writes, stages the file's
+// doubles: 138 a coarse column, the buffer holds 38 zds GR^2 values.
 static int import_history(dns_handle *h, const double *in) {
   const dns_geometry &g = h->g;
-  const size_t plane = (size_t)g.ny * g.nx, per = 2 * 23 * plane;
-  std::vector<double> tmp(3 * per);
-  for (int l = 0; l < 3; l++)
-    for (int w = 0; w < 2; w++)
-      for (int i = 0; i < g.nx; i++)
-        for (int j = 0; j < g.ny; j++)
-          for (int b = 0; b < 23; b++)
-            tmp[(((size_t)l * 2 + w) * 23 + b) * plane + (size_t)j * g.nx + i] =
-                in[((((size_t)l * 2 + w) * g.nx + i) * g.ny + j) * 23 + b];
-  if (is_f32(h)) {
-    std::vector<float> t32(3 * per);
-    for (size_t sl = 0; sl < 6; sl++)
-      for (size_t q = 0; q < plane; q++) tmp[sl * 23 * plane + q] -= 1.0;
-    for (size_t q = 0; q < t32.size(); q++) t32[q] = (float)tmp[q];
-    CUDA_TRY(cudaMemcpyAsync(h->hist, t32.data(), 3 * per * 4, cudaMemcpyHostToDevice, h->stream));
-  } else {
-    CUDA_TRY(cudaMemcpyAsync(h->hist, tmp.data(), 3 * per * 8, cudaMemcpyHostToDevice, h->stream));
-  }
+  double *stage = h->ff[1 - h->cur_f];
+  CUDA_TRY(cudaMemcpyAsync(stage, in, 138ull * g.nx * g.ny * 8, cudaMemcpyHostToDevice, h->stream));
+  launch_history(stage, h->hist, is_f32(h), g.nx, g.ny, h->stream);
+  CUDA_TRY(cudaGetLastError());
   CUDA_TRY(cudaStreamSynchronize(h->stream));
   h->hn = 0;
   h->hp = 1;

@@ -220,6 +220,7 @@ void launch_wall_plane(double *aos, double *wall, long long nodes, int nz, int k
 // an x range is one contiguous run of it
 void launch_soa_to_aos(const double *soa, double *aos, int nx, int ny, int P, int p0, int np, int nz_aos,
                        int k0_aos, cudaStream_t stream, int i0 = 0, int i1 = -1);
+void launch_history(const double *in, void *hist, bool f32, int nx, int ny, cudaStream_t stream);
 void launch_aos_to_soa(const double *aos, double *soa, int nx, int ny, int P, int p0, int np, int nz_aos,
                        int k0_aos, cudaStream_t stream, int i0 = 0, int i1 = -1);
 
