@@ -111,7 +111,7 @@ __device__ __forceinline__ int profile_of(const TkeArgs &A, int l, int k) {
 // to every thread of the block on return; kSumThreads threads.
 constexpr int kSumChunk = 512, kSumThreads = 160;
 template <int NF>
-struct SumSmem {
+struct alignas(16) SumSmem {  // read in 16-byte pairs
   // rows two banks apart: the adding lanes read the same position of NF rows
   double buf[2][NF][kSumChunk + 2];
 };
@@ -119,6 +119,7 @@ struct SumSmem {
 template <int NF, class Value>
 __device__ __forceinline__ void ordered_sums(SumSmem<NF> &S, size_t n, Value value, double *out) {
   static_assert(NF <= 32, "one lane a sequence");
+  static_assert(alignof(SumSmem<NF>) >= 16 && (kSumChunk + 2) % 2 == 0, "every row starts on 16 bytes");
   constexpr int W = kSumThreads - 32, PER = kSumChunk / W;
   const int t0 = (int)threadIdx.x - 32, lane = threadIdx.x & 31;
   auto produce = [&](size_t base, int b) {
