@@ -84,7 +84,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     fine_pair_kernel(const double *__restrict__ src, double *__restrict__ dst, const double *__restrict__ mid,
                      const int8_t *__restrict__ wf, Dims d, PairGrid g, double om, const DevState *st,
                      double *__restrict__ part, double *__restrict__ wpart) {
-  extern __shared__ double M[];
+  extern __shared__ __align__(16) double M[];  // bulk copies land in it
   constexpr int kTX = 32 * NS, kPlane = kRing * kTX;
   const int zds = d.zds, zdf = d.zdf, gr = d.gr, nx = d.nxf, ny = d.nyf;
   const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);  // warp-uniform
