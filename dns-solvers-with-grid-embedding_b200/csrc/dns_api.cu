@@ -100,7 +100,7 @@ struct dns_handle {
   size_t tke_ws_bytes = 0;
   double *tke_wall = nullptr;          // planar fields of the two wall planes [2][4][nyf][nxf]
   long tke_wall_gen = -1;              // wall_gen they were made from
-  unsigned int *fin_counter = nullptr; // finalize's block counter and log row
+  unsigned int *fin_counter = nullptr; // finalize's block counter and log row; a two-substep pass gave up
   cudaStream_t aux = nullptr;          // fine substeps and injection (lowest priority)
   cudaEvent_t ev_start = nullptr, ev_inj = nullptr, ev_fine[4] = {}, ev_if[4] = {};
   cudaEvent_t ev_xfer[kXferChunks] = {};  // one per x run of a level transfer
@@ -1184,12 +1184,13 @@ static void L_fine(dns_handle *h, int src, int dst, bool first, bool last, bool 
 static void L_fine_pair(dns_handle *h, int src, int dst, int m, bool first, bool last, cudaStream_t st) {
   const size_t mid = (size_t)m * 2 * 19 * h->d.nyf * h->d.nxf;
   double *part = h->partials + h->pl.fine, *wpart = h->partials + h->pl.wall;
+  unsigned int *lost = h->fin_counter + 2;
   if (is_f32(h))
     launch_fine_pair_f32(F(h->ff[src]), F(h->ff[dst]), F(h->iface_mid) + mid, h->wflag, h->d, h->shape.pair,
-                         h->g.omega_f, h->state, part, wpart, first, last, st);
+                         h->g.omega_f, h->state, part, wpart, lost, first, last, st);
   else
     launch_fine_pair_f64(h->ff[src], h->ff[dst], h->iface_mid + mid, h->wflag, h->d, h->shape.pair, h->g.omega_f,
-                         h->state, part, wpart, first, last, st);
+                         h->state, part, wpart, lost, first, last, st);
 }
 // Interface planes of substep it: those of the fine buffer fbuf, or (fbuf < 0)
 // slot m of the planes between two substeps of a pass
@@ -1517,7 +1518,13 @@ extern "C" int dns_step(dns_handle *h, long ncoarse, dns_step_log *log) {
       }
       // wshearstr.c:139-143 aborts on NaN only; an infinite stress is logged and the run goes on
       if (status == DNS_OK && std::isnan(r.stress)) {
-        status = fail(DNS_ENAN, "NaN wall shear stress at step " + std::to_string(ss0 + q));
+        unsigned int lost = 0;
+        CUDA_TRY(cudaMemcpyAsync(&lost, h->fin_counter + 2, 4, cudaMemcpyDeviceToHost, h->stream));
+        CUDA_TRY(cudaStreamSynchronize(h->stream));
+        const std::string at = std::to_string(ss0 + q);
+        status = lost ? fail(DNS_ECUDA, "a wait of the two-substep kernel ran out in step " + at +
+                                            " or before it: the state is not valid")
+                      : fail(DNS_ENAN, "NaN wall shear stress at step " + at);
       }
     }
     done += n;

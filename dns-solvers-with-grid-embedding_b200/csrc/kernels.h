@@ -84,14 +84,15 @@ bool pairs_pay_f32(const Dims &d, const PairGrid &g);
 int prepare_pair_f64();
 // two substeps from src into dst; mid: the interface planes between them,
 // [2 walls][19][nyf][nxf]; part: per-block flow-rate pairs [2 g.blocks()] (last);
-// wpart: per-block wall-shear pairs [6][g.blocks()] (first)
+// wpart: per-block wall-shear pairs [6][g.blocks()] (first); lost: set, and never
+// cleared, where a wait of the kernel ran out (dst is not valid)
 int prepare_pair_f32();
 void launch_fine_pair_f32(const float *src, float *dst, const float *mid, const int8_t *wflag, const Dims &d,
-                          const PairGrid &g, double om, const DevState *st, double *part, double *wpart, bool first,
-                          bool last, cudaStream_t stream);
+                          const PairGrid &g, double om, const DevState *st, double *part, double *wpart,
+                          unsigned int *lost, bool first, bool last, cudaStream_t stream);
 void launch_fine_pair_f64(const double *src, double *dst, const double *mid, const int8_t *wflag, const Dims &d,
-                          const PairGrid &g, double om, const DevState *st, double *part, double *wpart, bool first,
-                          bool last, cudaStream_t stream);
+                          const PairGrid &g, double om, const DevState *st, double *part, double *wpart,
+                          unsigned int *lost, bool first, bool last, cudaStream_t stream);
 
 
 // record a message for dns_last_error() on the calling thread (dns_api.cu)
@@ -145,7 +146,8 @@ void launch_inject_f64(const double *fsrc, double *cdst, const Dims &d, const La
 // pair_first / pair_last: the step's first / last fine pass took two substeps
 // (it left the wall-shear / flow-rate partials by its own tiles)
 // log: the rows of a group of steps; counter[1] is the next row, counter[0] the
-// kernel's block count (0 between launches)
+// kernel's block count (0 between launches); a row's wall stress is NaN where
+// counter[2] is set (a two-substep pass gave up)
 void launch_finalize(DevState *st, DevLog *log, double *partials, unsigned int *counter,
                      const PartialLayout &pl, const Dims &d, const LaunchShape &s, const StepParams &sp,
                      bool pair_first, bool pair_last, cudaStream_t stream);

@@ -769,7 +769,7 @@ __global__ void __launch_bounds__(NT) finalize2_kernel(DevState *st, DevLog *lg,
   // lanes 0..4: flow rate, lower and upper wall shear, momentum, mass
   const double *S = sh, *U = sh + 6;  // (U, D) pairs per plane: lower k=1,2,3, upper zdf-2,-3,-4
   const double m0 = st->momentum, d0 = st->denst, f0 = st->force;
-  const unsigned int at_row = counter[1];
+  const unsigned int at_row = counter[1], lost = counter[2];
   double num, den, fac = 1.;
   if (lane == 0) {
     num = m0 * a.flow_scale;
@@ -800,7 +800,7 @@ __global__ void __launch_bounds__(NT) finalize2_kernel(DevState *st, DevLog *lg,
     r.flowrate = q;
     r.stup = stup;
     r.stdown = stdown;
-    r.stress = 0.5 * (stup + stdown);
+    r.stress = lost ? __longlong_as_double(0x7ff8000000000000LL) : 0.5 * (stup + stdown);
     r.pgrad = f0 * a.pgrad_scale;
     lg[at_row] = r;
     counter[1] = at_row + 1;

@@ -12,7 +12,7 @@ template <int MODE>
 __global__ void __launch_bounds__(32 * kPairMaxZds, 1)
     fine_pair_f32(const float *__restrict__ src, float *__restrict__ dst, const float *__restrict__ mid,
                   const int8_t *__restrict__ wf, Dims d, PairGrid g, float om, const DevState *st,
-                  double *__restrict__ part, double *__restrict__ wpart) {
+                  double *__restrict__ part, double *__restrict__ wpart, unsigned int *__restrict__ lost) {
   extern __shared__ __align__(16) float Mf[];
   __shared__ PairSync S;
   const int nblk = gridDim.x * gridDim.y, blk = blockIdx.y * gridDim.x + blockIdx.x;
@@ -35,6 +35,7 @@ __global__ void __launch_bounds__(32 * kPairMaxZds, 1)
   P.part = part + ((size_t)blockIdx.z * nblk + blk) * 2;
   P.wpart = wpart + (size_t)blk * 2;
   P.wstride = (size_t)nblk * 2;
+  P.lost = lost;
   pair_tile<MODE>(Mf, S, P);
 }
 
@@ -68,16 +69,16 @@ int prepare_pair_f32() {
 }
 
 void launch_fine_pair_f32(const float *src, float *dst, const float *mid, const int8_t *wflag, const Dims &d,
-                          const PairGrid &g, double om, const DevState *st, double *part, double *wpart, bool first,
-                          bool last, cudaStream_t stream) {
+                          const PairGrid &g, double om, const DevState *st, double *part, double *wpart,
+                          unsigned int *lost, bool first, bool last, cudaStream_t stream) {
   const dim3 grid(g.ntx, g.nly, 2), block(32 * d.zds);
   const size_t smem = pair_smem_f32(d.zds);
   const float omf = (float)om;
   switch ((last ? 1 : 0) | (first ? 2 : 0)) {
-    case 0: fine_pair_f32<0><<<grid, block, smem, stream>>>(src, dst, mid, wflag, d, g, omf, st, part, wpart); break;
-    case 1: fine_pair_f32<1><<<grid, block, smem, stream>>>(src, dst, mid, wflag, d, g, omf, st, part, wpart); break;
-    case 2: fine_pair_f32<2><<<grid, block, smem, stream>>>(src, dst, mid, wflag, d, g, omf, st, part, wpart); break;
-    default: fine_pair_f32<3><<<grid, block, smem, stream>>>(src, dst, mid, wflag, d, g, omf, st, part, wpart); break;
+    case 0: fine_pair_f32<0><<<grid, block, smem, stream>>>(src, dst, mid, wflag, d, g, omf, st, part, wpart, lost); break;
+    case 1: fine_pair_f32<1><<<grid, block, smem, stream>>>(src, dst, mid, wflag, d, g, omf, st, part, wpart, lost); break;
+    case 2: fine_pair_f32<2><<<grid, block, smem, stream>>>(src, dst, mid, wflag, d, g, omf, st, part, wpart, lost); break;
+    default: fine_pair_f32<3><<<grid, block, smem, stream>>>(src, dst, mid, wflag, d, g, omf, st, part, wpart, lost); break;
   }
 }
 

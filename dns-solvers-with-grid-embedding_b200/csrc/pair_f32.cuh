@@ -130,6 +130,7 @@ struct PairSync {
   unsigned long long pushed[kPairMaxZds], taken[kPairMaxZds], staged[kPairMaxZds], middle[kPairMaxZds];
   unsigned long long solid[kMaxRun + 4];
   double sums[kPairMaxZds][4];
+  int stop;
 };
 
 struct PairTile {
@@ -142,6 +143,7 @@ struct PairTile {
   const int8_t *wf;
   double *part, *wpart;       // this tile's flow-rate pair; wall-shear pairs of row r at wpart[r * wstride]
   size_t wstride;
+  unsigned int *lost;         // set where a wait ran out
 };
 
 // One tile and run of one fine block.  MODE bits: 1 flow-rate partials, 2
@@ -162,6 +164,7 @@ __device__ __forceinline__ void pair_tile(float *M, PairSync &S, const PairTile 
   const int nb = bulk ? (x0 + cnt < nx ? npair + 1 : n1) : 0;
   const bool alone = lane >= nb && lane < npair;
   if (threadIdx.x == 0) {
+    S.stop = 0;
     for (int w = 0; w < zds; w++) {
       const int n = 1 + (w > 0) + (w < zds - 1), arrivals = (bulk ? 1 : 0) + max(0, npair - nb);
       mb_init(&S.pushed[w], n);
@@ -223,7 +226,7 @@ __device__ __forceinline__ void pair_tile(float *M, PairSync &S, const PairTile 
     const unsigned nodeb = (unsigned)p * planeb + (unsigned)x * 4u;
     const float om = P.om, Gf = P.Gf;
     double acc[2] = {0., 0.}, wacc[2] = {0., 0.};
-    bool ok = true;
+    bool gone = false;  // a wait of the block ran out
     f2 f[19], k0 = 0, p0 = 0;  // population 0 of rows t and t - 1
     // (every lane has collided the rows' old values; the fence puts the reads before
     // the copies, which go by another way to shared memory)
@@ -246,14 +249,16 @@ __device__ __forceinline__ void pair_tile(float *M, PairSync &S, const PairTile 
     auto next = [&](int y) { return y == ny - 1 ? 0 : y + 1; };
     int y = P.y0 == 0 ? ny - 1 : P.y0 - 1;  // row t = 0
     int yd = y;                             // the row that substep 2 takes (t - 1)
-    int s3 = 0;                             // t mod 3
+    int t = 0, s3 = 0;                      // s3: t mod 3
     auto first_half = [&](int t1, int ahead) {
-      if (t1 <= L + 1) ok = mb_wait(&S.staged[warp], t1 & 1) && ok;
+      if (t1 <= L + 1) mb_wait(&S.staged[warp], t1 & 1, &S.stop);
 #pragma unroll
       for (int a = 0; a < 19; a++) f[a] = reinterpret_cast<const f2 *>(Sw + a * 64)[lane];
+      const int halt = *(volatile int *)&S.stop;
       const Mac2 m = collide2(f, om, Gf);
       pin2(f);
-      if (t1 <= L) stage(ahead);
+      gone = __any_sync(0xffffffffu, halt);
+      if (t1 <= L && !gone) stage(ahead);
       if ((MODE & 2) && wall_sum_plane && t1 >= 1 && t1 <= L) {
         if (own0) wacc[0] += (double)lo2(m.u0);
         if (own1) wacc[0] += (double)hi2(m.u0);
@@ -265,12 +270,12 @@ __device__ __forceinline__ void pair_tile(float *M, PairSync &S, const PairTile 
     };
     stage(y);
     first_half(0, next(y));
-    for (int t = 0; t <= L + 1; t++) {
+    for (; !gone && t <= L + 1; t++) {
       const int yn = next(y);
       const int r2c = (t & 1) * 64, r2p = 64 - r2c;
       const int r3c = s3 * 64, r3n = (s3 == 2 ? 0 : s3 + 1) * 64, r3p = (s3 == 0 ? 2 : s3 - 1) * 64;
       // the pushes along x store aligned pairs, one value from the lane beside
-      if (t > 0) ok = mb_wait(&S.taken[q], (t - 1) & 1) && ok;
+      if (t > 0) mb_wait(&S.taken[q], (t - 1) & 1, &S.stop);
       {
         auto slot = [&](int a, int row) {
           const int r = ring_depth(a) == 1 ? 0
@@ -312,9 +317,10 @@ __device__ __forceinline__ void pair_tile(float *M, PairSync &S, const PairTile 
         }
       }
       mb_arrive(S.pushed, lane, q, zds);
-      ok = mb_wait(&S.pushed[q], t & 1) && ok;
+      mb_wait(&S.pushed[q], t & 1, &S.stop);
       f2 h[19];
-      if (iface && t >= 2) ok = mb_wait(&S.middle[warp], t & 1) && ok;  // row t - 1, the copies' (t - 2)nd phase
+      // row t - 1, the copies' (t - 2)nd phase
+      if (iface && t >= 2) mb_wait(&S.middle[warp], t & 1, &S.stop);
 #pragma unroll
       for (int a = 1; a < 19; a++)
         h[a] = *reinterpret_cast<const f2 *>(
@@ -323,7 +329,7 @@ __device__ __forceinline__ void pair_tile(float *M, PairSync &S, const PairTile 
       mb_arrive(S.taken, lane, q, zds);
       const Mac2 m = collide2(h, om, Gf);
       pin2(h);
-      if (iface && t >= 1 && t <= L)  // the interface row that substep 2 takes next (row t)
+      if (iface && t >= 1 && t <= L && !*(volatile int *)&S.stop)  // the interface row that substep 2 takes next (row t)
         copy(Mq - c0, P.mid + ((size_t)(upper ? 19 : 0) * ny + y) * nx, plane, &S.middle[warp]);
       const bool now = t >= 2;
       const bool o0 = own0 && now, o1 = own1 && now;
@@ -418,7 +424,11 @@ __device__ __forceinline__ void pair_tile(float *M, PairSync &S, const PairTile 
       y = yn;
       s3 = s3 == 2 ? 0 : s3 + 1;
     }
-    if (!ok) acc[0] = wacc[0] = __longlong_as_double(0x7ff8000000000000LL);  // the step reports a NaN wall stress
+    if (gone) {
+      *P.lost = 1u;
+      drain(&S.staged[warp], min(t, L + 1));
+      if (iface) drain(&S.middle[warp], min(t - 1, L) - 1);
+    }
     if (MODE) {
       double v[4] = {acc[0], acc[1], wacc[0], wacc[1]};
 #pragma unroll

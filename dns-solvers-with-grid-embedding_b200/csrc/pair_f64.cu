@@ -83,7 +83,7 @@ template <int MODE, int NS>
 __global__ void __launch_bounds__(kPairThreads, 1)
     fine_pair_kernel(const double *__restrict__ src, double *__restrict__ dst, const double *__restrict__ mid,
                      const int8_t *__restrict__ wf, Dims d, PairGrid g, double om, const DevState *st,
-                     double *__restrict__ part, double *__restrict__ wpart) {
+                     double *__restrict__ part, double *__restrict__ wpart, unsigned int *__restrict__ lost) {
   extern __shared__ __align__(16) double M[];  // bulk copies land in it
   constexpr int kTX = 32 * NS, kPlane = kRing * kTX;
   const int zds = d.zds, zdf = d.zdf, gr = d.gr, nx = d.nxf, ny = d.nyf;
@@ -139,7 +139,9 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   const unsigned nodeb = (unsigned)p * planeb + (unsigned)x * 8u;  // byte offset of (plane, x) in a population
   __shared__ unsigned long long pushed[kPairMaxZds], taken[kPairMaxZds], staged[kPairMaxZds], middle[kPairMaxZds];
   __shared__ unsigned long long solid[kMaxRun + 4];
+  __shared__ int stop;
   if (threadIdx.x == 0) {
+    stop = 0;
     for (int w = 0; w < zds; w++) {
       const int n = (1 + (w > 0) + (w < zds - 1)) * NS;
       mb_init(&pushed[w], n);
@@ -168,7 +170,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   }
   fence_async_proxy();
   __syncthreads();
-  bool ok = true;
+  bool gone = false;  // a wait of the block ran out
   double f[19], k0 = 0., p0 = 0.;  // population 0 of rows t and t - 1
   // the warp's columns of a row of 19 populations (stride apart) into rows
   // `pitch` apart: lane a copies population a.  (Every lane has collided the rows'
@@ -191,16 +193,18 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   auto next = [&](int y) { return y == ny - 1 ? 0 : y + 1; };
   int y = y0 == 0 ? ny - 1 : y0 - 1;  // row t = 0
   int yd = y;                         // the row that substep 2 takes (t - 1)
-  int s3 = 0;                         // t mod 3
+  int t = 0, s3 = 0;                  // s3: t mod 3
   // substep 1 of row t1 (the y index of the row after it: ahead), up to the collision
   auto first_half = [&](int t1, int ahead) {
-    if (t1 <= L + 1) ok = mb_wait(&staged[warp], t1 & 1) && ok;
+    if (t1 <= L + 1) mb_wait(&staged[warp], t1 & 1, &stop);
 #pragma unroll
     for (int a = 0; a < 19; a++) f[a] = Sq[a * 32];
+    const int halt = *(volatile int *)&stop;
     double dens, u0, u1, u2;
     collide_pairs_f64(f, om, Gf, dens, u0, u1, u2);
     pin(f);
-    if (t1 <= L) stage(ahead);
+    gone = __any_sync(0xffffffffu, halt);
+    if (t1 <= L && !gone) stage(ahead);
     if ((MODE & 2) && own && t1 >= 1 && t1 <= L) {
       if (wall_sum_plane) wacc[0] += u0;
       if (wall_rho_plane) wacc[1] += dens;
@@ -208,12 +212,12 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   };
   stage(y);
   first_half(0, next(y));
-  for (int t = 0; t <= L + 1; t++) {
+  for (; !gone && t <= L + 1; t++) {
     const int yn = next(y);
     // rows t - 1, t, t + 1 in the two- and three-row rings
     const int r2c = (t & 1) * kTX, r2p = kTX - r2c;
     const int r3c = s3 * kTX, r3n = (s3 == 2 ? 0 : s3 + 1) * kTX, r3p = (s3 == 0 ? 2 : s3 - 1) * kTX;
-    if (t > 0) ok = mb_wait(&taken[q], (t - 1) & 1) && ok;
+    if (t > 0) mb_wait(&taken[q], (t - 1) & 1, &stop);
     {
       // where a push of population a from row t lands: row t + e_y, or t itself for a bounce
       auto slot = [&](int a, int row) {
@@ -246,10 +250,10 @@ __global__ void __launch_bounds__(kPairThreads, 1)
       }
     }
     mb_arrive(pushed, lane, q, zds);
-    ok = mb_wait(&pushed[q], t & 1) && ok;
+    mb_wait(&pushed[q], t & 1, &stop);
     double h[19];
     // the interface row: row t - 1, the copies' (t - 2)nd phase
-    if (iface && t >= 2) ok = mb_wait(&middle[warp], t & 1) && ok;
+    if (iface && t >= 2) mb_wait(&middle[warp], t & 1, &stop);
 #pragma unroll
     for (int a = 1; a < 19; a++)
       h[a] = Mr[iface ? a * kTX : ring_off(a) * kTX + (ring_depth(a) == 1 ? 0 : (ring_depth(a) == 2 ? r2p : r3p))];
@@ -258,7 +262,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     double dens, u0, u1, u2;
     collide_pairs_f64(h, om, Gf, dens, u0, u1, u2);
     pin(h);
-    if (iface && t >= 1 && t <= L)  // the interface row that substep 2 takes next (row t)
+    if (iface && t >= 1 && t <= L && !*(volatile int *)&stop)  // the interface row that substep 2 takes next (row t)
       copy(Mq - lane, kTX, mid + ((size_t)(upper ? 19 : 0) * ny + y) * nx, plane, &middle[warp]);
     if (t >= 2 && own) {
       if ((MODE & 1) && unit) {
@@ -311,7 +315,11 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     y = yn;
     s3 = s3 == 2 ? 0 : s3 + 1;
   }
-  if (!ok) acc[0] = wacc[0] = __longlong_as_double(0x7ff8000000000000LL);  // the step reports a NaN wall stress
+  if (gone) {
+    *lost = 1u;
+    drain(&staged[warp], min(t, L + 1));
+    if (iface) drain(&middle[warp], min(t - 1, L) - 1);
+  }
   __syncthreads();
   // partials in a fixed order: lanes by shuffles, then the warps in order
   const int nblk = gridDim.x * gridDim.y, blk = blockIdx.y * gridDim.x + blockIdx.x;
@@ -397,13 +405,13 @@ int prepare_pair_f64() {
 }
 
 void launch_fine_pair_f64(const double *src, double *dst, const double *mid, const int8_t *wflag, const Dims &d,
-                          const PairGrid &g, double om, const DevState *st, double *part, double *wpart, bool first,
-                          bool last, cudaStream_t stream) {
+                          const PairGrid &g, double om, const DevState *st, double *part, double *wpart,
+                          unsigned int *lost, bool first, bool last, cudaStream_t stream) {
   const dim3 grid(g.ntx, g.nly, 2), block(32 * d.zds * g.ns);
   const size_t smem = pair_smem(d.zds, g.ns);
 #define PAIR_CASE(M, N) \
   case M * 2 + N - 1:   \
-    fine_pair_kernel<M, N><<<grid, block, smem, stream>>>(src, dst, mid, wflag, d, g, om, st, part, wpart); break;
+    fine_pair_kernel<M, N><<<grid, block, smem, stream>>>(src, dst, mid, wflag, d, g, om, st, part, wpart, lost); break;
   switch (((last ? 1 : 0) | (first ? 2 : 0)) * 2 + g.ns - 1) {
     PAIR_CASE(0, 1) PAIR_CASE(1, 1) PAIR_CASE(2, 1) PAIR_CASE(3, 1)
     PAIR_CASE(0, 2) PAIR_CASE(1, 2) PAIR_CASE(2, 2) PAIR_CASE(3, 2)

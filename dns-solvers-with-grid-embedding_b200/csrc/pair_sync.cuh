@@ -25,8 +25,9 @@ constexpr int kMaxRun = 256;  // rows of a run (the wall flags of a run are kept
 
 // Split barriers, one a plane: its warps and those of the planes beside it arrive
 // (only they push into its rows, and only it reads them), its warps wait for the
-// phase.  The waits are bounded: false after some 10 ms, which only a fault of
-// these files could cause (every warp makes the same arrivals).
+// phase.  The waits are bounded: kTries attempts, 1.5 us each where the phase does not
+// complete, so about 0.1 s, which only a fault of these files could take (every warp
+// makes the same arrivals).
 __device__ __forceinline__ void mb_init(unsigned long long *b, int count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"((unsigned)__cvta_generic_to_shared(b)), "r"(count)
                : "memory");
@@ -42,18 +43,23 @@ __device__ __forceinline__ void mb_arrive(unsigned long long *b, int lane, int q
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"((unsigned)__cvta_generic_to_shared(b + n))
                  : "memory");
 }
-__device__ __forceinline__ bool mb_wait(unsigned long long *b, int parity) {
+// Where they run out, or find the block's stop set, stop is set and the warp goes on
+// to the end of its row, where it reads stop: a vote and a branch at every wait cost
+// 10% of the two-substep pass.
+constexpr int kTries = 1 << 16;
+__device__ __forceinline__ void mb_wait(unsigned long long *b, int parity, volatile int *stop, int tries = kTries) {
   const unsigned a = (unsigned)__cvta_generic_to_shared(b);
-  for (int n = 0; n < (1 << 16); n++) {
+  for (int n = 0; n < tries; n++) {
     unsigned ok;
     asm volatile(
         "{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
         : "=r"(ok)
         : "r"(a), "r"(parity)
         : "memory");
-    if (ok) return true;
+    if (ok) return;
+    if (*stop) break;
   }
-  return false;
+  *stop = 1;
 }
 
 // Bulk copies into a warp's rows: the warp's barrier completes when `bytes` have landed.
@@ -79,6 +85,16 @@ __device__ __forceinline__ void lane_copies_arrive(unsigned long long *b) {
                : "memory");
 }
 __device__ __forceinline__ void fence_async_proxy() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
+
+// A warp that reads stop takes no further row and issues no further copy: the launch
+// is reported in *lost (the step's log row and every later one carry a NaN wall
+// stress, dns_step returns an error), and the warp's own copies land before it leaves:
+// phases up to `copies` of its barrier b (the last one may not have been issued).
+__device__ __forceinline__ void drain(unsigned long long *b, int copies) {
+  int none = 0;
+  for (int c = max(copies - 1, 0); c <= copies; c++) mb_wait(b, c & 1, &none, 4096);
+  asm volatile("cp.async.wait_all;\n" ::: "memory");
+}
 
 // a thread-uniform base plus a 32-bit byte offset (population arrays are below 4 GB)
 template <class T>

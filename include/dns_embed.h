@@ -192,7 +192,9 @@ int dns_get_force(dns_handle *h, double *force);
    ftcdtransfer, exchange/fexchange.  log (may be NULL) receives ncoarse rows.
    Returns DNS_ENAN if a wall shear stress is NaN (the reference calls
    MPI_Abort on isnan, wshearstr.c:139-143; an infinite stress is logged and
-   stepping goes on, as there); the state is then left as computed. */
+   stepping goes on, as there); the state is then left as computed.  Returns
+   DNS_ECUDA where a two-substep kernel gave up waiting inside (the wall stress is
+   then NaN as well); the state is not valid, and the handle says so from then on. */
 int dns_step(dns_handle *h, long ncoarse, dns_step_log *log);
 
 /* ---- statistics ---------------------------------------------------------- */

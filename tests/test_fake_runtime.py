@@ -1,0 +1,78 @@
+"""The channel driver's host code on a stand-in for the CUDA runtime (no GPU): what the
+calls return where the device reports a failure or memory runs out, and what is
+launched.  Each test runs its statements in a child process with fake_cudart.c
+preloaded; `rt` there is the stand-in, `channel` makes a channel."""
+from __future__ import annotations
+
+import os
+import subprocess
+import sys
+import textwrap
+
+import pytest
+
+from conftest import PKG_NAME, ROOT
+
+PRELUDE = f"""
+import ctypes, importlib
+import numpy as np
+rt = ctypes.CDLL(None)
+rt.fake_limit.argtypes = [ctypes.c_size_t]
+rt.fake_used.restype = ctypes.c_size_t
+for f in ("fake_launches", "fake_graph_launches", "fake_instantiated"):
+    getattr(rt, f).restype = ctypes.c_long
+pkg = importlib.import_module("{PKG_NAME}")
+def params(xdv, ydv, zdv, zds, gr, precision="FP64", **kw):
+    return pkg.make_params(xdv=xdv, ydv=ydv, zdv=zdv, zds=zds, gratio=gr, Rebs=200.0, CFL=2.0, pattern=None,
+                           precision=getattr(pkg, precision), forcing=pkg.FORCING_CONST, force_const=1e-5, **kw)
+def channel(*a, **kw):
+    return pkg.Channel(params(*a, **kw))
+def error(call):
+    try:
+        call()
+    except pkg.DnsError as e:
+        return e
+    return None
+"""
+
+
+@pytest.fixture(scope="session")
+def fake(tmp_path_factory):
+    so = tmp_path_factory.mktemp("fake") / "fake_cudart.so"
+    subprocess.run(["gcc", "-shared", "-fPIC", "-O1", "-Wall", "-Werror", str(ROOT / "tests" / "fake_cudart.c"), "-o",
+                    str(so)], check=True)
+
+    def run(code):
+        r = subprocess.run([sys.executable, "-c", PRELUDE + textwrap.dedent(code)], cwd=ROOT, capture_output=True,
+                           text=True, timeout=300, env=dict(os.environ, LD_PRELOAD=str(so)))
+        assert r.returncode == 0, r.stderr[-3000:]
+
+    return run
+
+
+@pytest.mark.parametrize("precision", ["FP64", "FP32"])
+def test_a_wait_that_ran_out_is_an_error_of_its_own(fake, precision):
+    """A two-substep pass that gave up sets a word that stays set: the step's row has a
+    NaN wall stress and dns_step says what happened, in that call and in later ones."""
+    fake(f"""
+    with channel(8, 5, 7, 5, 2, precision="{precision}") as ch:
+        ch.set_fine_pairs(1)
+        ch.step(4)
+        assert rt.fake_launches(b"fine_pair") == 4
+        rt.fake_lost(1)
+        for _ in range(2):
+            e = error(lambda: ch.step(1))
+            assert e is not None and e.code == pkg.DNS_ECUDA and "wait" in str(e), e
+            rt.fake_lost(0)
+    """)
+
+
+def test_a_nan_wall_stress_without_it_stays_what_it_was(fake):
+    fake("""
+    with channel(8, 5, 7, 5, 2) as ch:
+        rt.fake_stress(ctypes.c_double(float("inf")))
+        assert error(lambda: ch.step(2)) is None
+        rt.fake_stress(ctypes.c_double(float("nan")))
+        e = error(lambda: ch.step(2))
+        assert e is not None and e.code == pkg.DNS_ENAN and "NaN" in str(e), e
+    """)
