@@ -227,6 +227,15 @@ __global__ void __launch_bounds__(256) record_fields(const T *__restrict__ soa, 
       for (int a = 0; a < 19; a++) g[a] = population<T>(f + (size_t)a * stride, a);
       double dens, mx, my, mz;
       moments_f64(g, dens, mx, my, mz);
+      if (!isfinite(dens)) {  // 0 f of the definition's sums is not 0 where f is not finite
+        mx = my = mz = 0.;
+#pragma unroll
+        for (int a = 0; a < 19; a++) {
+          mx += (double)ex_of(a) * g[a];
+          my += (double)ey_of(a) * g[a];
+          mz += (double)ez_of(a) * g[a];
+        }
+      }
       tile[0][r][tx] = mx / dens;
       tile[1][r][tx] = my / dens;
       tile[2][r][tx] = mz / dens;
