@@ -1180,6 +1180,10 @@ static void L_fine(dns_handle *h, int src, int dst, bool first, bool last, bool 
     launch_fine_f64(h->ff[src], h->ff[dst], h->wflag, h->d, h->shape, h->g.omega_f, h->state, h->partials, h->pl,
                     first, last, stats, st);
 }
+static void L_fine_stats(dns_handle *h, int src, cudaStream_t st) {
+  if (is_f32(h)) launch_fine_stats_f32(F(h->ff[src]), h->d, h->shape, h->partials, h->pl, st);
+  else launch_fine_stats_f64(h->ff[src], h->d, h->shape, h->partials, h->pl, st);
+}
 // Two substeps in one pass; m: slot of the interface planes between them
 static void L_fine_pair(dns_handle *h, int src, int dst, int m, bool first, bool last, cudaStream_t st) {
   const size_t mid = (size_t)m * 2 * 19 * h->d.nyf * h->d.nxf;
@@ -1353,11 +1357,12 @@ extern "C" int dns_load_uniform(dns_handle *h, const char *dir, int cntr) {
 struct Pass {
   int first, n, m;  // first substep, substeps, slot of the planes between them
 };
-static int plan_passes(const dns_handle *h, bool sample, Pass *out) {
+// The passes of a step, sampled or not: sampling leaves the run as it is (the sums
+// behind a constant flow rate's force, and FP32 roundings, go by the passes).
+static int plan_passes(const dns_handle *h, Pass *out) {
   int n = 0, m = 0;
   for (int s = 1; s <= h->d.gr;) {
-    // the statistics of a sampled step are summed by the one-substep kernel
-    const bool two = pairs_on(h) && s < h->d.gr && !(sample && s == 1);
+    const bool two = pairs_on(h) && s < h->d.gr;
     out[n++] = Pass{s, two ? 2 : 1, two ? m++ : -1};
     s += two ? 2 : 1;
   }
@@ -1373,12 +1378,15 @@ static void issue_step(dns_handle *h, cudaStream_t S, bool sample) {
   };
   const int nc = 1 - h->cur_c;
   Pass P[4];
-  const int np = plan_passes(h, sample, P);
+  const int np = plan_passes(h, P);
   signal(h->ev_start, S, T);
   PROFILED(h, 0, L_coarse(h, h->cur_c, nc, sample, S));
   rotate_history(h);
   PROFILED(h, 1, L_extract(h, nc, h->hn, S));
   int cur = h->cur_f;
+  // the statistics are of the state before the step: a pass of one substep sums them as
+  // it reads it, before one of two they are summed by themselves
+  if (sample && P[0].n == 2) PROFILED(h, 6, L_fine_stats(h, cur, T));
   for (int i = 0; i < np; i++) {
     const int nf = 1 - cur, last = P[i].first + P[i].n - 1;
     auto transfer = [&] {
@@ -1413,7 +1421,7 @@ static void issue_step(dns_handle *h, cudaStream_t S, bool sample) {
   signal(h->ev_inj, T, S);
   PROFILED(h, 5, launch_finalize(h->state, h->dlog, h->partials, h->fin_counter, h->pl, d, h->shape, h->sp,
                                  P[0].n == 2, P[np - 1].n == 2, S));
-  if (sample) PROFILED(h, 6, launch_stats_finalize(h->stats_acc, h->partials, h->pl, d, h->shape, S));
+  if (sample) PROFILED(h, 6, launch_stats_finalize(h->stats_acc, h->partials, h->pl, d, h->shape, P[0].n == 2, S));
   h->cur_f = cur;
   h->cur_c = nc;
 }

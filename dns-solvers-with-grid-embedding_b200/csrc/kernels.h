@@ -124,6 +124,13 @@ void launch_extract_f64(const double *fc, double *hist_n, const Dims &d, const L
 void launch_fine_f64(const double *src, double *dst, const int8_t *wflag, const Dims &d, const LaunchShape &s,
                      double om, const DevState *st, double *partials, const PartialLayout &pl, bool first,
                      bool last, bool stats, cudaStream_t stream);
+// plane statistics of the stored fine state, into the partials of a sampled step (one
+// whose first pass takes two substeps; else fine's stats does it), kStatRows rows a block
+constexpr int kStatRows = 8;
+void launch_fine_stats_f64(const double *src, const Dims &d, const LaunchShape &s, double *partials,
+                           const PartialLayout &pl, cudaStream_t stream);
+void launch_fine_stats_f32(const float *src, const Dims &d, const LaunchShape &s, double *partials,
+                           const PartialLayout &pl, cudaStream_t stream);
 // The interface transfers of n substeps (at most 4), two launches: macroscopic
 // fields into mac[substep - 1][2 walls][4][nyf][nxf], then one block per (tile,
 // substep, wall, population) into the substep's planes
@@ -151,8 +158,9 @@ void launch_inject_f64(const double *fsrc, double *cdst, const Dims &d, const La
 void launch_finalize(DevState *st, DevLog *log, double *partials, unsigned int *counter,
                      const PartialLayout &pl, const Dims &d, const LaunchShape &s, const StepParams &sp,
                      bool pair_first, bool pair_last, cudaStream_t stream);
+// own_pass: the fine partials are launch_fine_stats's
 void launch_stats_finalize(double *acc, const double *partials, const PartialLayout &pl, const Dims &d,
-                           const LaunchShape &s, cudaStream_t stream);
+                           const LaunchShape &s, bool own_pass, cudaStream_t stream);
 // direct encalc2 reduction of the stored state into st (momentum, denst, force)
 void launch_flow_sums_f64(const double *fc, const double *ff, DevState *st, double *partials,
                           const PartialLayout &pl, const Dims &d, const LaunchShape &s, const StepParams &sp,

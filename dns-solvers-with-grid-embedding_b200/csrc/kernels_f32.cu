@@ -150,6 +150,25 @@ __global__ void __launch_bounds__(kThreads, KIND ? DNS_F32_BULK_MINB : 0) fine_f
   if (MODE & 4) block_reduce_stat(sacc, spart + blk * kStatPart);
 }
 
+// the statistics of a sampled step whose first pass takes two substeps (kernels_f64.cu)
+__global__ void __launch_bounds__(kThreads) fine_stats_f32(const float *__restrict__ src, Dims d,
+                                                          double *__restrict__ spart) {
+  const int nx = d.nxf, ny = d.nyf, i = blockIdx.x * blockDim.x + threadIdx.x;
+  const size_t pstride = (size_t)2 * d.zds * ny * nx;
+  PlaneStat sacc;
+  sacc.init();
+  for (int r = 0; r < kStatRows; r++) {
+    const int j = blockIdx.y * kStatRows + r;
+    if (i >= nx || j >= ny) break;
+    float f[19];
+    load19f(src, ((size_t)blockIdx.z * ny + j) * nx + i, pstride, f);
+    const Mac32 m = macro_f32(f);
+    sacc.add(m.u0, m.u1, m.u2, 1.0 + (double)m.drho);
+  }
+  const size_t blk = ((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+  block_reduce_stat(sacc, spart + blk * kStatPart);
+}
+
 // ------------------------------------------------------------------ four nodes per thread
 // The stream-collide of one channel with the batched engine's four-node
 // threads (quad_f32.cuh: 16-byte loads and stores, opposite populations
@@ -653,6 +672,12 @@ void launch_fine_f32(const float *src, float *dst, const int8_t *wflag, const Di
     FINE32_CASE(7)
   }
 #undef FINE32_CASE
+}
+
+void launch_fine_stats_f32(const float *src, const Dims &d, const LaunchShape &s, double *partials,
+                           const PartialLayout &pl, cudaStream_t stream) {
+  fine_stats_f32<<<dim3(s.fgx, (d.nyf + kStatRows - 1) / kStatRows, 2 * d.zds), s.bx, 0, stream>>>(
+      src, d, partials + pl.stats_f);
 }
 
 void launch_interface_f32(const float *hn, const float *hp, const float *hpp, float *corner, const IfaceTarget &tg,

@@ -249,6 +249,34 @@ __global__ void __launch_bounds__(kMaxThreads, DNS_MINB_FINE) fine_kernel(const 
   if (MODE & 4) block_reduce_stat(sacc, spart + blk * kStatPart);
 }
 
+// The plane statistics of fine_kernel's MODE 4 in a pass of their own: for steps whose
+// first pass takes two substeps, which are taken alike whether they are sampled or not.
+// Eight rows a thread: the block's merge, not HBM, bounds it (256x128x83, 638 MB: 147 us
+// with fine_kernel's two rows, 117 us this way).  A step of that channel sampled every
+// time takes 703 us (819 us when a sampled step's substeps went one by one), one of
+// 130x120x40 at ratio 3 831 us (804).
+__global__ void __launch_bounds__(kMaxThreads) fine_stats_kernel(const double *__restrict__ src, Dims d,
+                                                                double *__restrict__ spart) {
+  const int nx = d.nxf, ny = d.nyf, i = blockIdx.x * blockDim.x + threadIdx.x;
+  const size_t pstride = (size_t)2 * d.zds * ny * nx;
+  PlaneStat sacc;
+  sacc.init();
+  const int j0 = blockIdx.y * kStatRows, rows = i < nx ? min(kStatRows, ny - j0) : 0;
+  const double *at = src + ((size_t)blockIdx.z * ny + j0) * nx + i;
+  double f[19], next[19];
+  if (rows) load19(at, 0, pstride, next);
+  for (int r = 0; r < rows; r++) {  // the next row's loads are on their way meanwhile
+#pragma unroll
+    for (int a = 0; a < 19; a++) f[a] = next[a];
+    if (r + 1 < rows) load19(at, (size_t)(r + 1) * nx, pstride, next);
+    double dens, mx, my, mz;
+    moments_f64(f, dens, mx, my, mz);
+    sacc.add(mx / dens, my / dens, mz / dens, dens);
+  }
+  const size_t blk = ((size_t)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+  block_reduce_stat(sacc, spart + blk * kStatPart);
+}
+
 // ------------------------------------------------------------------ interface
 // Coarse-to-fine transfer for one substep, both walls (tinterpolate_hrmt.c,
 // derivative.c, bcucof_opt.c, ctfdtransfer_opt.c): Hermite interpolation in
@@ -1085,6 +1113,12 @@ void launch_fine_f64(const double *src, double *dst, const int8_t *wflag, const 
 #undef FINE_CASE
 }
 
+void launch_fine_stats_f64(const double *src, const Dims &d, const LaunchShape &s, double *partials,
+                           const PartialLayout &pl, cudaStream_t stream) {
+  fine_stats_kernel<<<dim3(s.fgx, (d.nyf + kStatRows - 1) / kStatRows, 2 * d.zds), s.bx, 0, stream>>>(
+      src, d, partials + pl.stats_f);
+}
+
 void launch_interface_f64(const double *hn, const double *hp, const double *hpp, double *mac, const IfaceTarget *tg,
                           int n, const Dims &d, const LaunchShape &s, double omega_c, double omega_f,
                           cudaStream_t stream) {
@@ -1171,14 +1205,14 @@ void launch_finalize(DevState *st, DevLog *log, double *partials, unsigned int *
 }
 
 void launch_stats_finalize(double *acc, const double *partials, const PartialLayout &pl, const Dims &d,
-                           const LaunchShape &s, cudaStream_t stream) {
+                           const LaunchShape &s, bool own_pass, cudaStream_t stream) {
   StatsArgs a;
   a.nzp = 2 * d.zdf + d.nzc - 4;
   a.zdf = d.zdf;
   a.nzc = d.nzc;
   a.zds = d.zds;
   a.bc = s.n_coarse_blocks();
-  a.bf = s.n_fine_blocks();
+  a.bf = own_pass ? (long)s.fgx * ((d.nyf + kStatRows - 1) / kStatRows) : s.n_fine_blocks();
   a.nc = (double)d.nx * d.ny;
   a.nf = (double)d.nxf * d.nyf;
   stats_finalize_kernel<<<a.nzp, 256, 0, stream>>>(acc, partials + pl.stats_c, partials + pl.stats_f, a);

@@ -200,7 +200,8 @@ int dns_step(dns_handle *h, long ncoarse, dns_step_log *log);
 /* ---- statistics ---------------------------------------------------------- */
 /* Every `every` coarse steps (0 = off) the pre-step state is sampled on the
    device: per plane of the composite profile (statistics.c:48-146 plane order)
-   FP64 sums of u, v, w, rho and their second moments are accumulated. */
+   FP64 sums of u, v, w, rho and their second moments are accumulated.  The steps are
+   the same, bit for bit, whether they are sampled or not. */
 int dns_set_sampling(dns_handle *h, long every);
 int dns_stats_reset(dns_handle *h);
 /* Accumulated profiles, out[DNS_NSTAT][nz_profile], samples in *nsamples:
