@@ -94,8 +94,9 @@ struct dns_handle {
   DevLog *dlog = nullptr;              // kLogCap rows
   DevLog *hlog = nullptr;              // pinned mirror
   double *stats_acc = nullptr;         // [nz_profile][kStatRow] running statistics
-  double *iface_mac = nullptr;         // FP64: interface rho, u [GR][2][4][nyf][nxf]; FP32: corner data
-  double *iface_mid = nullptr;         // interface planes between the substeps of a pass [GR / 2][2][19][nyf][nxf]
+  double *iface_mac = nullptr;         // FP64: interface rho, u [2][4][nyf][nxf]; FP32: corner data
+  double *iface_mid = nullptr;         // interface planes between the substeps of a pass [GR / 2][2][19][nyf][nxf],
+                                       // FP64 then their rho, u [GR / 2][2][4][nyf][nxf]
   void *tke_ws = nullptr;              // statistics / budget work space (allocated on first use)
   size_t tke_ws_bytes = 0;
   double *tke_wall = nullptr;          // planar fields of the two wall planes [2][4][nyf][nxf]
@@ -136,15 +137,38 @@ static bool pairs_on(const dns_handle *h) {
   return h->shape.pair.on() && (h->pairs < 0 ? pairs_pay(h->p, h->d, h->shape.pair) : h->pairs > 0);
 }
 
-// what the passes of two substeps need beyond the single ones
+// Bytes that the passes of two substeps need beyond the single ones: the interface
+// planes between the substeps of each, FP64 also rho, u at the nodes of those planes
+// (one launch makes them with the first pass's last ones).
+static size_t pair_bytes(const dns_params &p, const dns_geometry &g) {
+  const size_t fplane = (size_t)g.nyf * g.nxf;
+  return (g.gr / 2) * fplane * (p.precision == DNS_FP32 ? 2 * 19 * 4ull : (2 * 19 + 2 * 4) * 8ull);
+}
 static int ready_pairs(dns_handle *h) {
   if (h->iface_mid) return DNS_OK;
-  const size_t bytes = (h->g.gr / 2) * 2ull * 19 * h->g.nyf * h->g.nxf * (h->p.precision == DNS_FP32 ? 4 : 8);
   if (h->p.precision == DNS_FP32 ? prepare_pair_f32() : prepare_pair_f64())
     return fail(DNS_ECUDA, "shared-memory limit of the two-substep kernels");
-  if (cudaMalloc((void **)&h->iface_mid, bytes) != cudaSuccess)
+  if (cudaMalloc((void **)&h->iface_mid, pair_bytes(h->p, h->g)) != cudaSuccess) {
+    cudaGetLastError();
     return fail(DNS_ENOMEM, "interface planes between two substeps");
+  }
   return DNS_OK;
+}
+
+// Device memory for a call on a handle.  What is left goes to the work that cannot do
+// without: if need be the planes of the two-substep passes go, and the fine substeps
+// are taken one at a time from then on.
+static cudaError_t call_alloc(dns_handle *h, void **ptr, size_t bytes) {
+  cudaError_t e = cudaMalloc(ptr, bytes);
+  if (e == cudaErrorMemoryAllocation && h->iface_mid) {
+    cudaGetLastError();
+    drop_graphs(h);
+    h->pairs = 0;
+    cudaFree(h->iface_mid);
+    h->iface_mid = nullptr;
+    e = cudaMalloc(ptr, bytes);
+  }
+  return e;
 }
 
 // Bracket one launch with events when profiling; returns the pair index or -1.
@@ -315,9 +339,9 @@ extern "C" int dns_geometry_of(const dns_params *p, dns_geometry *g) {
   PartialLayout pl = partial_layout(d, s);
   const long long nc = 19LL * g->nzc * g->ny * g->nx, nf = 19LL * 2 * p->zds * g->nyf * g->nxf;
   const long long esz = p->precision == DNS_FP32 ? 4 : 8;  // bytes per stored population
-  const long long mac = esz == 4 ? 2LL * 23 * g->ny * g->nx * 4 : 8LL * GR * g->nyf * g->nxf;  // elements of esz
-  const long long mid = pairs_pay(*p, d, s.pair) ? (GR / 2) * 2LL * 19 * g->nyf * g->nxf : 0;
-  g->device_bytes = esz * (2 * nc + 2 * nf + 3LL * 2 * 23 * g->ny * g->nx + mac + mid) +
+  const long long mac = esz == 4 ? 2LL * 23 * g->ny * g->nx * 4 : 8LL * g->nyf * g->nxf;  // elements of esz
+  g->device_bytes = (pairs_pay(*p, d, s.pair) ? (long long)pair_bytes(*p, *g) : 0) +
+                    esz * (2 * nc + 2 * nf + 3LL * 2 * 23 * g->ny * g->nx + mac) +
                     8 * (pl.total + (long long)kStatRow * g->nz_profile + 2LL * 19 * g->nyf * g->nxf) +
                     (long long)g->nyf * g->nxf + (long long)kLogCap * sizeof(DevLog) + sizeof(DevState);
   return DNS_OK;
@@ -404,13 +428,16 @@ extern "C" int dns_create(const dns_params *p, dns_handle **out) {
   size_t freeb = 0, totalb = 0;
   CUDA_TRY(cudaSetDevice(p->device));
   CUDA_TRY(cudaMemGetInfo(&freeb, &totalb));
-  if ((long long)freeb < g.device_bytes) return fail(DNS_ENOMEM, "not enough free device memory for this channel");
   dns_handle *h = new dns_handle();
   h->p = *p;
   h->g = g;
   h->d = Dims{g.nx, g.ny, g.nzc, g.nxf, g.nyf, g.zdf, p->zds, g.gr, g.nzs};
   h->shape = make_shape(h->d, p->precision == DNS_FP32);
   h->pl = partial_layout(h->d, h->shape);
+  if ((long long)freeb < g.device_bytes - (pairs_on(h) ? (long long)pair_bytes(*p, g) : 0)) {
+    delete h;
+    return fail(DNS_ENOMEM, "not enough free device memory for this channel");
+  }
   h->sp = StepParams{g.omega_c, g.omega_f, p->ub, p->force_const, p->forcing == DNS_FORCING_CFR ? 1 : 0, p->fltr, 0.0};
   // the FP32 form's mass partials sum deviations from w: add the weight sum once
   if (p->precision == DNS_FP32) h->sp.den_offset = encalc2_weight_sum(h->d);
@@ -436,20 +463,23 @@ extern "C" int dns_create(const dns_params *p, dns_handle **out) {
   if ((rc = alloc((void **)&h->dlog, kLogCap * sizeof(DevLog)))) return rc;
   if ((rc = alloc((void **)&h->stats_acc, (size_t)g.nz_profile * kStatRow * 8))) return rc;
   // FP64: interface rho, u at fine nodes; FP32: corner values and derivatives (float4)
-  const size_t mac_bytes = esz == 4 ? 2ull * 23 * g.ny * g.nx * 16 : 8ull * g.gr * g.nyf * g.nxf * esz;
+  const size_t mac_bytes = esz == 4 ? 2ull * 23 * g.ny * g.nx * 16 : 8ull * g.nyf * g.nxf * esz;
   if ((rc = alloc((void **)&h->iface_mac, mac_bytes))) return rc;
   if (p->fltr && (esz == 4 ? prepare_filter_f32() : prepare_filter_f64())) {
     dns_destroy(h);
     return fail(DNS_ECUDA, "shared-memory limit of the filtered injection");
   }
-  if (pairs_on(h) && (rc = ready_pairs(h))) {
-    dns_destroy(h);
-    return rc;
-  }
   if ((rc = alloc((void **)&h->fin_counter, 256))) return rc;
   cudaMemset(h->fin_counter, 0, 256);
   if ((rc = alloc((void **)&h->wall_dev, 2ull * g.nxf * g.nyf * 19 * 8))) return rc;
   cudaMemset(h->wall_dev, 0, 2ull * g.nxf * g.nyf * 19 * 8);
+  if (pairs_on(h) && (rc = ready_pairs(h))) {
+    if (rc != DNS_ENOMEM) {
+      dns_destroy(h);
+      return rc;
+    }
+    h->pairs = 0;  // the channel fits, their planes do not: single substeps
+  }
   if (cudaMallocHost((void **)&h->hlog, kLogCap * sizeof(DevLog)) != cudaSuccess) {
     dns_destroy(h);
     return fail(DNS_ENOMEM, "cudaMallocHost failed");
@@ -540,7 +570,7 @@ static int staging(dns_handle *h, int level, double **out) {
   }
   if (!h->stage) {
     const size_t n = std::max(level_doubles(h->g, 0), level_doubles(h->g, 1));
-    if (cudaMalloc(&h->stage, n * 8) != cudaSuccess) return fail(DNS_ENOMEM, "AoS staging buffer");
+    if (call_alloc(h, (void **)&h->stage, n * 8) != cudaSuccess) return fail(DNS_ENOMEM, "AoS staging buffer");
   }
   *out = h->stage;
   return DNS_OK;
@@ -940,8 +970,8 @@ extern "C" int dns_write_fields(dns_handle *h, const char *dir, int cntr) {
   const int zds = h->p.zds;
   const size_t nmax = std::max((size_t)g.nx * g.ny * g.nzc, (size_t)g.nxf * g.nyf * g.zdf);
   double *dvel = nullptr, *dden = nullptr;
-  if (cudaMalloc(&dvel, nmax * 3 * 8) != cudaSuccess) return fail(DNS_ENOMEM, "field staging");
-  if (cudaMalloc(&dden, nmax * 8) != cudaSuccess) {
+  if (call_alloc(h, (void **)&dvel, nmax * 3 * 8) != cudaSuccess) return fail(DNS_ENOMEM, "field staging");
+  if (call_alloc(h, (void **)&dden, nmax * 8) != cudaSuccess) {
     cudaFree(dvel);
     return fail(DNS_ENOMEM, "field staging");
   }
@@ -1018,7 +1048,7 @@ static int fields_planar(dns_handle *h, double *const q[3]) {
   // the host from the wall populations when those change, kept on the device
   const size_t npl = (size_t)g.nxf * g.nyf, lvl = level_nodes(g, 1);
   if (h->tke_wall_gen != h->wall_gen) {
-    if (!h->tke_wall && cudaMalloc(&h->tke_wall, 2 * 4 * npl * 8) != cudaSuccess)
+    if (!h->tke_wall && call_alloc(h, (void **)&h->tke_wall, 2 * 4 * npl * 8) != cudaSuccess)
       return fail(DNS_ENOMEM, "wall-plane fields for the budget");
     std::vector<double> wv(npl * 3), wd(npl), planes(2 * 4 * npl);
     for (int lv = 1; lv < 3; lv++) {
@@ -1061,7 +1091,7 @@ extern "C" int dns_tke_budget(dns_handle *h, double *prof, double *ufl, double *
     cudaFree(h->tke_ws);
     h->tke_ws = nullptr;
     h->tke_ws_bytes = 0;
-    if (cudaMalloc(&h->tke_ws, need) != cudaSuccess) return fail(DNS_ENOMEM, "field buffers for the budget");
+    if (call_alloc(h, &h->tke_ws, need) != cudaSuccess) return fail(DNS_ENOMEM, "field buffers for the budget");
     h->tke_ws_bytes = need;
   }
   double *q[3], *o = static_cast<double *>(h->tke_ws);
@@ -1219,9 +1249,13 @@ static void L_iface(dns_handle *h, const IfaceDest *to, int n, cudaStream_t st) 
     }
     return;
   }
-  for (int q = 0; q < n; q++) set(to[q].fbuf >= 0 ? h->ff[to[q].fbuf] : nullptr, h->iface_mid, tg[q], to[q]);
-  launch_interface_f64(h->hist + h->hn * hs, h->hist + h->hp * hs, h->hist + h->hpp * hs, h->iface_mac, tg, n, h->d,
-                       h->shape, h->g.omega_c, h->g.omega_f, st);
+  double *more = h->iface_mid ? h->iface_mid + (size_t)(h->d.gr / 2) * 2 * 19 * plane : nullptr;
+  for (int q = 0; q < n; q++) {
+    set(to[q].fbuf >= 0 ? h->ff[to[q].fbuf] : nullptr, h->iface_mid, tg[q], to[q]);
+    tg[q].mac = q == 0 ? h->iface_mac : more + (size_t)(q - 1) * 2 * 4 * plane;
+  }
+  launch_interface_f64(h->hist + h->hn * hs, h->hist + h->hp * hs, h->hist + h->hpp * hs, tg, n, h->d, h->shape,
+                       h->g.omega_c, h->g.omega_f, st);
 }
 static void L_inject(dns_handle *h, int fbuf, int cbuf, cudaStream_t st) {
   if (is_f32(h))
@@ -1279,8 +1313,8 @@ extern "C" int dns_load_uniform(dns_handle *h, const char *dir, int cntr) {
     cudaFree(lev);
     cudaFree(bad);
   };
-  if (cudaMalloc(&uni, nuni * 8) != cudaSuccess || cudaMalloc(&lev, nlev * 8) != cudaSuccess ||
-      cudaMalloc(&bad, sizeof(int)) != cudaSuccess) {
+  if (call_alloc(h, (void **)&uni, nuni * 8) != cudaSuccess || call_alloc(h, (void **)&lev, nlev * 8) != cudaSuccess ||
+      call_alloc(h, (void **)&bad, sizeof(int)) != cudaSuccess) {
     release();
     return fail(DNS_ENOMEM, "uniform-grid staging");
   }
@@ -1500,8 +1534,12 @@ extern "C" int dns_step(dns_handle *h, long ncoarse, dns_step_log *log) {
       long run = 1;  // steps from here on that are sampled like this one
       while (run < kGraphSteps && q + run < n && sampled(h->ss + run) == sample) run++;
       cudaGraphExec_t G = run == kGraphSteps && !h->prof.on ? step_graph(h, sample) : nullptr;
-      if (G) CUDA_TRY(cudaGraphLaunch(G, h->stream));
-      else
+      if (G && cudaGraphLaunch(G, h->stream) != cudaSuccess) {  // it may need memory at its first launch
+        cudaGetLastError();
+        h->graphs_ok = false;
+        G = nullptr;
+      }
+      if (!G)
         for (long r = 0; r < run; r++) issue_step(h, h->stream, sample);
       q += run;
       h->ss += run;

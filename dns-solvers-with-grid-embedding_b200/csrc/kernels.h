@@ -132,15 +132,16 @@ void launch_fine_stats_f64(const double *src, const Dims &d, const LaunchShape &
 void launch_fine_stats_f32(const float *src, const Dims &d, const LaunchShape &s, double *partials,
                            const PartialLayout &pl, cudaStream_t stream);
 // The interface transfers of n substeps (at most 4), two launches: macroscopic
-// fields into mac[substep - 1][2 walls][4][nyf][nxf], then one block per (tile,
+// fields into each one's mac[2 walls][4][nyf][nxf], then one block per (tile,
 // substep, wall, population) into the substep's planes
 struct IfaceTarget {
   int substep;
+  double *mac;    // FP64 form
   void *out[2];   // plane of population 0 of the lower / upper wall
   size_t stride;  // elements from one population's plane to the next
 };
-void launch_interface_f64(const double *hn, const double *hp, const double *hpp, double *mac, const IfaceTarget *tg,
-                          int n, const Dims &d, const LaunchShape &s, double omega_c, double omega_f,
+void launch_interface_f64(const double *hn, const double *hp, const double *hpp, const IfaceTarget *tg, int n,
+                          const Dims &d, const LaunchShape &s, double omega_c, double omega_f,
                           cudaStream_t stream);
 // filtered: the FLTR transfer (ftcdtransfer_lesfltr.c) instead of ftcdtransfer.c
 // (its kernels' shared-memory limit is raised first, on the current device)

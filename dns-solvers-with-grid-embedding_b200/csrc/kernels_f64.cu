@@ -305,7 +305,7 @@ struct IfaceArgs {
 // the substeps of one launch: blockIdx.z is ((substep * 2) + wall) * fields + field
 struct IfaceSet {
   IfaceArgs a[4];
-  int mac[4];  // slot of the macroscopic fields
+  double *mac[4];  // macroscopic fields [2 walls][4][nyf][nxf]
   double *out[4][2];
   size_t stride[4];
 };
@@ -406,12 +406,12 @@ __device__ __forceinline__ double iface_eval(const double (&cf)[16], int ii, int
 
 // Phase 1: macroscopic fields.  Block (tile, substep, wall, field b < 4) writes
 // field b (rho, ux, uy, uz) at the tile's fine interface nodes into
-// mac[substep][wall][b][j][i].
+// the substep's mac[wall][b][j][i].
 template <int GR>
 __global__ void __launch_bounds__(TPX *TPY) interface_macro_kernel(const double *__restrict__ hn,
                                                                    const double *__restrict__ hp,
                                                                    const double *__restrict__ hpp,
-                                                                   double *__restrict__ mac, Dims d, IfaceSet is) {
+                                                                   Dims d, IfaceSet is) {
   __shared__ IfaceSmem S;
   const int nx = d.nx, ny = d.ny, nxf = d.nxf, nyf = d.nyf;
   const int sub = blockIdx.z >> 3, w = (blockIdx.z >> 2) & 1, b = blockIdx.z & 3;
@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(TPX *TPY) interface_macro_kernel(const double 
   const int tx = threadIdx.x % TPX, ty = threadIdx.x / TPX;
   const size_t plane = (size_t)ny * nx, fplane = (size_t)nyf * nxf;
   iface_stage(S, hn, hp, hpp, ((size_t)w * 23 + b) * plane, i0, j0, nx, ny, ia);
-  double *o = mac + ((size_t)(is.mac[sub] * 2 + w) * 4 + b) * fplane;
+  double *o = is.mac[sub] + ((size_t)w * 4 + b) * fplane;
 #pragma unroll
   for (int q = 0; q < CPT; q++) {
     const int cx = tx + TPX * (q % (ITX / TPX)), cy = ty + TPY * (q / (ITX / TPX));
@@ -452,8 +452,7 @@ template <int GR>
 __global__ void __launch_bounds__(TPX *TPY) interface_pop_kernel(const double *__restrict__ hn,
                                                                  const double *__restrict__ hp,
                                                                  const double *__restrict__ hpp,
-                                                                 const double *__restrict__ mac, Dims d,
-                                                                 IfaceSet is) {
+                                                                 Dims d, IfaceSet is) {
   __shared__ IfaceSmem S;
   const int nx = d.nx, ny = d.ny, nxf = d.nxf, nyf = d.nyf;
   const int sub = blockIdx.z / 38, w = (blockIdx.z / 19) & 1, a = blockIdx.z % 19;
@@ -464,7 +463,7 @@ __global__ void __launch_bounds__(TPX *TPY) interface_pop_kernel(const double *_
   iface_stage(S, hn, hp, hpp, ((size_t)w * 23 + 4 + a) * plane, i0, j0, nx, ny, ia);
   const int cls = a == 0 ? 0 : (a <= 6 ? 1 : 2);
   const double wa = cls == 0 ? 1. / 3. : (cls == 1 ? 1. / 18. : 1. / 36.);
-  const double *m = mac + (size_t)(is.mac[sub] * 2 + w) * 4 * fplane;
+  const double *__restrict__ m = is.mac[sub] + (size_t)w * 4 * fplane;
   double *out = is.out[sub][w] + (size_t)a * is.stride[sub];
 #pragma unroll
   for (int q = 0; q < CPT; q++) {
@@ -1119,8 +1118,8 @@ void launch_fine_stats_f64(const double *src, const Dims &d, const LaunchShape &
       src, d, partials + pl.stats_f);
 }
 
-void launch_interface_f64(const double *hn, const double *hp, const double *hpp, double *mac, const IfaceTarget *tg,
-                          int n, const Dims &d, const LaunchShape &s, double omega_c, double omega_f,
+void launch_interface_f64(const double *hn, const double *hp, const double *hpp, const IfaceTarget *tg, int n,
+                          const Dims &d, const LaunchShape &s, double omega_c, double omega_f,
                           cudaStream_t stream) {
   IfaceSet is{};
   for (int q = 0; q < n; q++) {
@@ -1133,20 +1132,20 @@ void launch_interface_f64(const double *hn, const double *hp, const double *hpp,
     ia.h3 = -2. * tmp * tmp * tmp + 3. * tmp * tmp;
     ia.h4 = tmp * tmp * tmp - tmp * tmp;
     ia.fac = omega_c / ((double)d.gr * omega_f);
-    is.mac[q] = tg[q].substep - 1;
+    is.mac[q] = tg[q].mac;
     for (int w = 0; w < 2; w++) is.out[q][w] = static_cast<double *>(tg[q].out[w]);
     is.stride[q] = tg[q].stride;
   }
   dim3 gm(s.igx, s.igy, n * 2 * 4), gp(s.igx, s.igy, n * 2 * 19), block(TPX * TPY);
   if (d.gr == 2) {
-    interface_macro_kernel<2><<<gm, block, 0, stream>>>(hn, hp, hpp, mac, d, is);
-    interface_pop_kernel<2><<<gp, block, 0, stream>>>(hn, hp, hpp, mac, d, is);
+    interface_macro_kernel<2><<<gm, block, 0, stream>>>(hn, hp, hpp, d, is);
+    interface_pop_kernel<2><<<gp, block, 0, stream>>>(hn, hp, hpp, d, is);
   } else if (d.gr == 3) {
-    interface_macro_kernel<3><<<gm, block, 0, stream>>>(hn, hp, hpp, mac, d, is);
-    interface_pop_kernel<3><<<gp, block, 0, stream>>>(hn, hp, hpp, mac, d, is);
+    interface_macro_kernel<3><<<gm, block, 0, stream>>>(hn, hp, hpp, d, is);
+    interface_pop_kernel<3><<<gp, block, 0, stream>>>(hn, hp, hpp, d, is);
   } else {
-    interface_macro_kernel<4><<<gm, block, 0, stream>>>(hn, hp, hpp, mac, d, is);
-    interface_pop_kernel<4><<<gp, block, 0, stream>>>(hn, hp, hpp, mac, d, is);
+    interface_macro_kernel<4><<<gm, block, 0, stream>>>(hn, hp, hpp, d, is);
+    interface_pop_kernel<4><<<gp, block, 0, stream>>>(hn, hp, hpp, d, is);
   }
 }
 

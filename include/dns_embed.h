@@ -83,7 +83,8 @@ typedef struct dns_geometry {
   int utime;                /* coarse steps per unit time */
   double omega_c, omega_f;  /* relaxation rates as the reference computes them */
   long long updates_per_step; /* xdv ydv zdc + 2 GR (GR xdv)(GR ydv) zds */
-  long long device_bytes;   /* HBM the handle allocates */
+  long long device_bytes;   /* HBM the handle allocates; where only the planes of two-substep
+                               passes do not fit, it does without them */
 } dns_geometry;
 
 /* One coarse step's log values, computed on the pre-step state S_n exactly as

@@ -76,3 +76,80 @@ def test_a_nan_wall_stress_without_it_stays_what_it_was(fake):
         e = error(lambda: ch.step(2))
         assert e is not None and e.code == pkg.DNS_ENAN and "NaN" in str(e), e
     """)
+
+
+# planes between the substeps, and (FP64) rho and u there: what only pairs need
+PAIR_BYTES = "(gr // 2) * (gr * x) * (gr * y) * (2 * 19 * 4 if precision == 'FP32' else (2 * 19 + 2 * 4) * 8)"
+
+
+@pytest.mark.parametrize("form", [("FP64", 128, 128, 51, 16, 2), ("FP64", 64, 48, 20, 16, 4), ("FP32", 96, 80, 20, 10, 4)])
+def test_a_channel_that_fits_without_pairs_is_created(fake, form):
+    """Sizes that take two substeps a pass by default: where memory lacks for their
+    planes alone the channel takes its substeps one at a time, and it is refused only
+    where it does not fit at all."""
+    precision, *grid = form
+    fake(f"""
+    precision, (x, y, z, s, gr) = "{precision}", {tuple(grid)}
+    need = {PAIR_BYTES}
+    g = pkg.geometry(params(x, y, z, s, gr, precision))
+    with channel(x, y, z, s, gr, precision) as ch:
+        used = rt.fake_used()
+        assert used >= g.device_bytes - 4096
+        ch.step(2)
+        assert rt.fake_launches(b"fine_pair") > 0
+    pairs = rt.fake_launches(b"fine_pair")
+    for short in (1, need):
+        rt.fake_limit(used - short)
+        with channel(x, y, z, s, gr, precision) as ch:
+            ch.step(2)
+            assert rt.fake_launches(b"fine_pair") == pairs
+            e = error(lambda: ch.set_fine_pairs(1))
+            assert e is not None and e.code == pkg.DNS_ENOMEM
+            ch.step(2)
+            rt.fake_limit(1 << 36)
+            ch.set_fine_pairs(-1)
+            ch.step(2)
+            assert rt.fake_launches(b"fine_pair") > pairs
+            pairs = rt.fake_launches(b"fine_pair")
+        assert rt.fake_used() == 0
+    rt.fake_limit(used - need - 8192)
+    e = error(lambda: channel(x, y, z, s, gr, precision))
+    assert e is not None and e.code == pkg.DNS_ENOMEM
+    assert rt.fake_used() == 0
+    """)
+
+
+def test_pairs_make_room_for_a_call_that_needs_memory(fake):
+    fake(f"""
+    precision, (x, y, z, s, gr) = "FP32", (16, 16, 7, 8, 4)
+    need = {PAIR_BYTES}
+    with channel(x, y, z, s, gr, precision) as ch:
+        ch.set_fine_pairs(1)
+        ch.step(60)
+        stage = 19 * (gr * x) * (gr * y) * (s + 1) * 8
+        rt.fake_limit(rt.fake_used() + stage - need)
+        ch.export_state(1)
+        pairs = rt.fake_launches(b"fine_pair")
+        assert pairs > 0
+        ch.step(60)
+        assert rt.fake_launches(b"fine_pair") == pairs
+    with channel(x, y, z, s, gr, precision) as ch:
+        ch.set_fine_pairs(1)
+        rt.fake_limit(rt.fake_used() + stage - need - 1)
+        e = error(lambda: ch.export_state(1))
+        assert e is not None and e.code == pkg.DNS_ENOMEM
+    """)
+
+
+def test_steps_go_on_one_by_one_where_a_graph_cannot_be_launched(fake):
+    fake("""
+    with channel(8, 5, 7, 5, 2) as ch:
+        for _ in range(12):
+            ch.step(6)
+        assert rt.fake_graph_launches() > 0
+        rt.fake_fail_graph_launch(ctypes.c_long(1))
+        n = rt.fake_launches(b"finalize2")
+        for _ in range(3):
+            ch.step(6)
+        assert rt.fake_launches(b"finalize2") == n + 18
+    """)
