@@ -44,9 +44,10 @@ constexpr int kLogCap = 1024;
 // 345..362 / 345; host time below 1 us.  kGraphSteps is the period of the buffers
 // (two) and the history ring (three).  Recording takes 0.5 to 0.8 ms, as much as 8
 // (smallest channel) to 30 groups save, so a group is recorded when it is due for the
-// kGraphAfter-th time; kStepGraphs bounds them: the six states that steps can start a
-// group from, sampled or not.
-constexpr int kGraphSteps = 6, kStepGraphs = 12, kGraphAfter = 8;
+// kGraphAfter-th time; kStepGraphs bounds them: the states that steps can start a group
+// from (two coarse buffers, two fine ones, three history slots), sampled or not.  A run
+// comes through six of either; seeding or importing again may give it six others.
+constexpr int kGraphSteps = 6, kStepGraphs = 24, kGraphAfter = 8;
 // x runs per level transfer (state import / export): up to 8 of at least 2 MB each,
 // below which a copy and its transpose are launches only (a 150 KB level: 9 us in
 // one run, 60 us in eight)

@@ -153,3 +153,31 @@ def test_steps_go_on_one_by_one_where_a_graph_cannot_be_launched(fake):
             ch.step(6)
         assert rt.fake_launches(b"finalize2") == n + 18
     """)
+
+
+@pytest.mark.parametrize("pairs", [0, 1])
+def test_groups_of_every_start_state_get_their_graph(fake, pairs):
+    """Groups start from any of the two coarse buffers, the two fine ones and the three
+    history slots, sampled or not; steps that change which of them go together (a state
+    seeded again after an odd number of passes) find a place for their graphs too."""
+    fake(f"""
+    def groups(ch):
+        for sampling in (0, 1):
+            ch.set_sampling(sampling)
+            for start in range(6):
+                n = rt.fake_graph_launches()
+                for _ in range(9):
+                    ch.step(6)
+                assert rt.fake_graph_launches() > n, (sampling, start)
+                ch.step(1)
+    with channel(8, 5, 7, 5, 2) as ch:
+        ch.set_fine_pairs({1 - pairs})
+        ch.step(1)
+        ch.set_fine_pairs({pairs})
+        ch.step(1)
+        groups(ch)
+        ch.init_seeded(1)
+        groups(ch)
+        groups(ch)
+        assert rt.fake_instantiated() <= 24
+    """)

@@ -52,3 +52,25 @@ def test_statistics_of_pairs_are_those_of_single_substeps(pkg, grid):
             ch.step(9)
             out.append(ch.stats()[0])
     np.testing.assert_allclose(*out, rtol=0, atol=1e-14)
+
+
+@pytest.mark.parametrize("every", [7, 20])
+@pytest.mark.parametrize("precision", ["FP64", "FP32"])
+def test_sampled_groups_match_unsampled_single_steps(pkg, precision, every):
+    """Pairs at ratio 2, runs of sampled and plain steps: groups issued as graphs against
+    steps issued one by one without sampling."""
+    p = params_for(pkg, macros(16, 6, 7, 6, 2, "PSLIP"), "cfr")
+    p.precision = getattr(pkg, precision)
+    out = []
+    for sampled in (False, True):
+        with pkg.Channel(p) as ch:
+            ch.set_fine_pairs(1)
+            ch.init_seeded(4)
+            if sampled:
+                ch.set_sampling(every)
+                log = np.concatenate([ch.step(n) for n in (301, 1, 298)])
+            else:
+                log = np.concatenate([ch.step(1) for _ in range(600)])
+            out.append([ch.export_state(l) for l in range(3)] + [ch.export_history(), log])
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
