@@ -226,7 +226,7 @@ __device__ __forceinline__ void pair_tile(float *M, PairSync &S, const PairTile 
     const unsigned nodeb = (unsigned)p * planeb + (unsigned)x * 4u;
     const float om = P.om, Gf = P.Gf;
     double acc[2] = {0., 0.}, wacc[2] = {0., 0.};
-    bool gone = false;  // a wait of the block ran out
+    bool ok = true, gone = false;  // a wait of the block ran out
     f2 f[19], k0 = 0, p0 = 0;  // population 0 of rows t and t - 1
     // (every lane has collided the rows' old values; the fence puts the reads before
     // the copies, which go by another way to shared memory)
@@ -251,13 +251,12 @@ __device__ __forceinline__ void pair_tile(float *M, PairSync &S, const PairTile 
     int yd = y;                             // the row that substep 2 takes (t - 1)
     int t = 0, s3 = 0;                      // s3: t mod 3
     auto first_half = [&](int t1, int ahead) {
-      if (t1 <= L + 1) mb_wait(&S.staged[warp], t1 & 1, &S.stop);
+      if (t1 <= L + 1) ok = mb_wait(&S.staged[warp], t1 & 1, &S.stop) && ok;
 #pragma unroll
       for (int a = 0; a < 19; a++) f[a] = reinterpret_cast<const f2 *>(Sw + a * 64)[lane];
-      const int halt = *(volatile int *)&S.stop;
       const Mac2 m = collide2(f, om, Gf);
       pin2(f);
-      gone = __any_sync(0xffffffffu, halt);
+      gone = !__all_sync(0xffffffffu, ok);
       if (t1 <= L && !gone) stage(ahead);
       if ((MODE & 2) && wall_sum_plane && t1 >= 1 && t1 <= L) {
         if (own0) wacc[0] += (double)lo2(m.u0);
@@ -275,7 +274,7 @@ __device__ __forceinline__ void pair_tile(float *M, PairSync &S, const PairTile 
       const int r2c = (t & 1) * 64, r2p = 64 - r2c;
       const int r3c = s3 * 64, r3n = (s3 == 2 ? 0 : s3 + 1) * 64, r3p = (s3 == 0 ? 2 : s3 - 1) * 64;
       // the pushes along x store aligned pairs, one value from the lane beside
-      if (t > 0) mb_wait(&S.taken[q], (t - 1) & 1, &S.stop);
+      if (t > 0) ok = mb_wait(&S.taken[q], (t - 1) & 1, &S.stop) && ok;
       {
         auto slot = [&](int a, int row) {
           const int r = ring_depth(a) == 1 ? 0
@@ -317,10 +316,10 @@ __device__ __forceinline__ void pair_tile(float *M, PairSync &S, const PairTile 
         }
       }
       mb_arrive(S.pushed, lane, q, zds);
-      mb_wait(&S.pushed[q], t & 1, &S.stop);
+      ok = mb_wait(&S.pushed[q], t & 1, &S.stop) && ok;
       f2 h[19];
       // row t - 1, the copies' (t - 2)nd phase
-      if (iface && t >= 2) mb_wait(&S.middle[warp], t & 1, &S.stop);
+      if (iface && t >= 2) ok = mb_wait(&S.middle[warp], t & 1, &S.stop) && ok;
 #pragma unroll
       for (int a = 1; a < 19; a++)
         h[a] = *reinterpret_cast<const f2 *>(
@@ -329,7 +328,8 @@ __device__ __forceinline__ void pair_tile(float *M, PairSync &S, const PairTile 
       mb_arrive(S.taken, lane, q, zds);
       const Mac2 m = collide2(h, om, Gf);
       pin2(h);
-      if (iface && t >= 1 && t <= L && !*(volatile int *)&S.stop)  // the interface row that substep 2 takes next (row t)
+      // the interface row that substep 2 takes next (row t)
+      if (iface && t >= 1 && t <= L && __all_sync(0xffffffffu, ok))
         copy(Mq - c0, P.mid + ((size_t)(upper ? 19 : 0) * ny + y) * nx, plane, &S.middle[warp]);
       const bool now = t >= 2;
       const bool o0 = own0 && now, o1 = own1 && now;
@@ -425,6 +425,7 @@ __device__ __forceinline__ void pair_tile(float *M, PairSync &S, const PairTile 
       s3 = s3 == 2 ? 0 : s3 + 1;
     }
     if (gone) {
+      S.stop = 1;
       *P.lost = 1u;
       drain(&S.staged[warp], min(t, L + 1));
       if (iface) drain(&S.middle[warp], min(t - 1, L) - 1);

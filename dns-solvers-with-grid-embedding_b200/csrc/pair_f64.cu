@@ -170,7 +170,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   }
   fence_async_proxy();
   __syncthreads();
-  bool gone = false;  // a wait of the block ran out
+  bool ok = true, gone = false;  // a wait of the block ran out
   double f[19], k0 = 0., p0 = 0.;  // population 0 of rows t and t - 1
   // the warp's columns of a row of 19 populations (stride apart) into rows
   // `pitch` apart: lane a copies population a.  (Every lane has collided the rows'
@@ -196,14 +196,13 @@ __global__ void __launch_bounds__(kPairThreads, 1)
   int t = 0, s3 = 0;                  // s3: t mod 3
   // substep 1 of row t1 (the y index of the row after it: ahead), up to the collision
   auto first_half = [&](int t1, int ahead) {
-    if (t1 <= L + 1) mb_wait(&staged[warp], t1 & 1, &stop);
+    if (t1 <= L + 1) ok = mb_wait(&staged[warp], t1 & 1, &stop) && ok;
 #pragma unroll
     for (int a = 0; a < 19; a++) f[a] = Sq[a * 32];
-    const int halt = *(volatile int *)&stop;
     double dens, u0, u1, u2;
     collide_pairs_f64(f, om, Gf, dens, u0, u1, u2);
     pin(f);
-    gone = __any_sync(0xffffffffu, halt);
+    gone = !__all_sync(0xffffffffu, ok);
     if (t1 <= L && !gone) stage(ahead);
     if ((MODE & 2) && own && t1 >= 1 && t1 <= L) {
       if (wall_sum_plane) wacc[0] += u0;
@@ -217,7 +216,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     // rows t - 1, t, t + 1 in the two- and three-row rings
     const int r2c = (t & 1) * kTX, r2p = kTX - r2c;
     const int r3c = s3 * kTX, r3n = (s3 == 2 ? 0 : s3 + 1) * kTX, r3p = (s3 == 0 ? 2 : s3 - 1) * kTX;
-    if (t > 0) mb_wait(&taken[q], (t - 1) & 1, &stop);
+    if (t > 0) ok = mb_wait(&taken[q], (t - 1) & 1, &stop) && ok;
     {
       // where a push of population a from row t lands: row t + e_y, or t itself for a bounce
       auto slot = [&](int a, int row) {
@@ -250,10 +249,10 @@ __global__ void __launch_bounds__(kPairThreads, 1)
       }
     }
     mb_arrive(pushed, lane, q, zds);
-    mb_wait(&pushed[q], t & 1, &stop);
+    ok = mb_wait(&pushed[q], t & 1, &stop) && ok;
     double h[19];
     // the interface row: row t - 1, the copies' (t - 2)nd phase
-    if (iface && t >= 2) mb_wait(&middle[warp], t & 1, &stop);
+    if (iface && t >= 2) ok = mb_wait(&middle[warp], t & 1, &stop) && ok;
 #pragma unroll
     for (int a = 1; a < 19; a++)
       h[a] = Mr[iface ? a * kTX : ring_off(a) * kTX + (ring_depth(a) == 1 ? 0 : (ring_depth(a) == 2 ? r2p : r3p))];
@@ -262,7 +261,8 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     double dens, u0, u1, u2;
     collide_pairs_f64(h, om, Gf, dens, u0, u1, u2);
     pin(h);
-    if (iface && t >= 1 && t <= L && !*(volatile int *)&stop)  // the interface row that substep 2 takes next (row t)
+    // the interface row that substep 2 takes next (row t)
+    if (iface && t >= 1 && t <= L && __all_sync(0xffffffffu, ok))
       copy(Mq - lane, kTX, mid + ((size_t)(upper ? 19 : 0) * ny + y) * nx, plane, &middle[warp]);
     if (t >= 2 && own) {
       if ((MODE & 1) && unit) {
@@ -316,6 +316,7 @@ __global__ void __launch_bounds__(kPairThreads, 1)
     s3 = s3 == 2 ? 0 : s3 + 1;
   }
   if (gone) {
+    stop = 1;
     *lost = 1u;
     drain(&staged[warp], min(t, L + 1));
     if (iface) drain(&middle[warp], min(t - 1, L) - 1);

@@ -43,11 +43,11 @@ __device__ __forceinline__ void mb_arrive(unsigned long long *b, int lane, int q
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];\n" ::"r"((unsigned)__cvta_generic_to_shared(b + n))
                  : "memory");
 }
-// Where they run out, or find the block's stop set, stop is set and the warp goes on
-// to the end of its row, where it reads stop: a vote and a branch at every wait cost
-// 10% of the two-substep pass.
+// False for a lane whose wait ran out or found the block's stop set: its warp goes on to
+// the middle of its row and leaves there.  (A vote and a branch at every wait cost 10% of
+// the two-substep pass, one a row 1.4%.)
 constexpr int kTries = 1 << 16;
-__device__ __forceinline__ void mb_wait(unsigned long long *b, int parity, volatile int *stop, int tries = kTries) {
+__device__ __forceinline__ bool mb_wait(unsigned long long *b, int parity, volatile int *stop, int tries = kTries) {
   const unsigned a = (unsigned)__cvta_generic_to_shared(b);
   for (int n = 0; n < tries; n++) {
     unsigned ok;
@@ -56,10 +56,10 @@ __device__ __forceinline__ void mb_wait(unsigned long long *b, int parity, volat
         : "=r"(ok)
         : "r"(a), "r"(parity)
         : "memory");
-    if (ok) return;
+    if (ok) return true;
     if (*stop) break;
   }
-  *stop = 1;
+  return false;
 }
 
 // Bulk copies into a warp's rows: the warp's barrier completes when `bytes` have landed.
@@ -86,9 +86,9 @@ __device__ __forceinline__ void lane_copies_arrive(unsigned long long *b) {
 }
 __device__ __forceinline__ void fence_async_proxy() { asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory"); }
 
-// A warp that reads stop takes no further row and issues no further copy: the launch
-// is reported in *lost (the step's log row and every later one carry a NaN wall
-// stress, dns_step returns an error), and the warp's own copies land before it leaves:
+// A warp that leaves sets stop, takes no further row and issues no further copy.  The
+// launch is reported in *lost: the step's log row and every later one carry a NaN wall
+// stress, and dns_step returns an error.  The warp's own copies land before it goes:
 // phases up to `copies` of its barrier b (the last one may not have been issued).
 __device__ __forceinline__ void drain(unsigned long long *b, int copies) {
   int none = 0;
