@@ -1470,7 +1470,8 @@ static void drop_graphs(dns_handle *h) {
 // The FP32 form's quad kernels at ratio 3 and 4 on larger channels go one by one:
 // us a step, one by one and from a graph, 96x64x40 at ratio 3 (2.9 M node updates)
 // 170.6 / 172.6, 96x64x50 at ratio 4 (8.2 M) 298 / 303, but 75x45x31 (1.4 M) 147 / 123
-// and 48x32x30 at ratio 4 (1.6 M) 116 / 115.
+// and 48x32x30 at ratio 4 (1.6 M) 116 / 115.  Why the graph is the slower one there has
+// not been found; the line is drawn by these figures alone.
 static bool groups_pay(const dns_handle *h) {
   const Dims &d = h->d;
   const long updates = 2L * d.gr * d.zds * d.nyf * d.nxf + (long)d.nx * d.ny * d.nzc;

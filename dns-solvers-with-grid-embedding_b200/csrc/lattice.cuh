@@ -146,7 +146,9 @@ __device__ __forceinline__ void collide_f64(double (&f)[19], double om, double G
 // m / d from y = 1 / d correctly rounded: two residual corrections of m y with
 // fused multiply-adds.  The last one rounds correctly by Markstein's theorem
 // (IBM J. Res. Dev. 34, 1990): the value it corrects is a faithful rounding of
-// the quotient.  Not for non-finite operands.
+// the quotient.  Not for non-finite operands, and not for |m| below 2^-968 (but 0),
+// where the residual underflows; momenta of populations near their weights are 0 or
+// above 2^-64.
 __device__ __forceinline__ double quotient_f64(double m, double d, double y) {
   double q = m * y;
   q = fma(fma(-q, d, m), y, q);

@@ -51,8 +51,10 @@ PairGrid make_pair_grid_f32(const Dims &d) {
 }
 
 // The single substeps of the FP32 form run at 88% of the HBM rate beside their
-// interface transfers; pairs, bound by issue, pay where a step has two of them and
-// its transfers go out together: GR 4.  Measured us per step, pairs against single
+// interface transfers.  A pair takes 204 us on 256x128x83 where two of them take 222,
+// at 36% of the HBM rate and 52% of the issue slots: latency, at the 16 warps that its
+// shared rows and registers leave an SM.  All its transfers stand in front of it, so it
+// pays where a step has two of them and the transfers go out together: GR 4.  Measured us per step, pairs against single
 // substeps: GR 4, zds 16: 637 MB 799 / 986, zds 10: 199 MB 410 / 425, 112 MB
 // 290 / 260; GR 2, zds 16: 319 MB 349 / 346, zds 8: 160 MB 272 / 248.
 bool pairs_pay_f32(const Dims &d, const PairGrid &g) {

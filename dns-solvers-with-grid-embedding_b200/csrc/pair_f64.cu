@@ -39,8 +39,8 @@
 // coarse-to-fine transfer (mid), its rows by bulk copies too.  Pushes into the
 // interface plane are dropped in both substeps, as in the one-substep kernel.
 //
-// 256x128x83 (two blocks of 512 x 256 x 16): 299 us for both substeps, 4.3 TB/s of
-// state; as two launches of the one-substep kernel 210 + 221 us, 5.9 TB/s.  Bound by
+// 256x128x83 (two blocks of 512 x 256 x 16): 308 us for both substeps, 4.1 TB/s of
+// state; as two launches of the one-substep kernel 435 us, 5.9 TB/s.  Bound by
 // FP64 issue and latency: a row of 16 planes takes 8 thousand cycles, of which the
 // FP64 pipe needs 4.2; HBM at the copy rate would take 195 us.
 //
@@ -388,7 +388,8 @@ PairGrid make_pair_grid(const Dims &d) {
 // against single substeps: GR 2, zds 16: 80 MB 122 / 116, 120 MB 144 / 165,
 // 159 MB 169 / 186, 638 MB 564 / 683; zds 12: 60 MB 113 / 102, 478 MB 522 / 571;
 // zds 8: 80 MB 142 / 138, 319 MB 425 / 459; GR 3, zds 9: 222 MB 426 / 409; GR 4,
-// zds 10: 149 MB 342 / 347, 398 MB 797 / 840.
+// zds 10: 149 MB 342 / 347, 398 MB 797 / 840.  (The line does not see the ratio: at
+// GR 4, where pairs also save transfers, the first of these lies 1.4% on its wrong side.)
 bool pairs_pay_f64(const Dims &d, const PairGrid &g) {
   const double w = 16. / (d.zds * g.ns), mb = 2. * d.zds * d.nyf * d.nxf * 19 * 8 * 1e-6;
   return g.on() && mb >= 100. * w * w;

@@ -224,13 +224,15 @@ int dns_plane_stats(dns_handle *h, double *out9xnz);
    the reference times only the whole loop, main :1252/:1377).  Classes:
    0 coarse stream-collide, 1 interface extraction, 2 fine stream-collide,
    3 coarse-to-fine interface, 4 fine-to-coarse injection, 5 reduction finalize,
-   6 statistics finalize.  Times accumulate until profiling is switched on again. */
+   6 statistics (finalize, and the fine level's own pass before a two-substep pass).  Times accumulate until profiling is switched on again. */
 #define DNS_NKERNEL 7
 int dns_set_profiling(dns_handle *h, int on);
 int dns_kernel_times(dns_handle *h, double *ms, long *launches);
 /* Fine substeps taken two at a time, in one pass over the fine state (zds <= 16
    and an even GR xdv): -1 where the state is large enough to gain by it
-   (default), 0 never, 1 wherever possible.  The state is the same either way. */
+   (default), 0 never, 1 wherever possible.  FP64 with a constant force: the same state
+   bit for bit either way; with a constant flow rate the force differs by the order of a
+   sum (1e-16 relative a step), and the FP32 form rounds in another grouping. */
 int dns_set_fine_pairs(dns_handle *h, int mode);
 
 /* ---- allocation-free reduction ------------------------------------------- */
